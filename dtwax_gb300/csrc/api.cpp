@@ -41,6 +41,7 @@ struct Shape {
   int grid = 0;   // CTAs
   int64_t items = 0;  // work items (while tuning: the candidate's chunk factor per mille)
   bool nh = false;  // narrow halo strips (FP16 pairs, narrow chunks)
+  bool deal = false;  // items go to the CTAs in turn instead of first come, first served
 };
 
 // Buffers of one batch that may be in flight on its own stream.
@@ -50,7 +51,7 @@ struct BatchCtx {
   cudaEvent_t done = nullptr;
   cudaEvent_t sweep_beg = nullptr, sweep_end = nullptr;  // bracket the last sweep launch
   bool sweep_timed = false;
-  DevBuf raw, query, meta, keys, results, seam, flags;
+  DevBuf raw, query, meta, keys, results, seam, flags, halo_read;
   HostBuf h_raw, h_meta, h_results, h_flags;
   int64_t seam_bytes = 0;
   bool meta_pending = false;
@@ -214,9 +215,10 @@ int choose_chunk_strips(int64_t strips_per_read, int64_t n_tasks, double mean_ro
   const double halo = (mean_rows + WH) / (2.0 * W) * (WH < W ? 1.1 : 1.0);
   double best_t = 1e300;
   int best_g = (int)strips_per_read;
-  for (int64_t g = 1; g <= strips_per_read; ++g) {
-    const int64_t chunks = (strips_per_read + g - 1) / g;
-    if (g > 1 && chunks == (strips_per_read + (g - 1) - 1) / (g - 1)) continue;
+  int64_t chunks = 0;
+  // the narrowest chunk of every chunk count
+  for (int64_t g = 1; g <= strips_per_read; g = chunks > 1 ? (strips_per_read + chunks - 2) / (chunks - 1) : g + 1) {
+    chunks = (strips_per_read + g - 1) / g;
     const int64_t items = n_tasks * chunks;
     const double waves = std::ceil((double)items / (double)total_warps);
     const double cost = (double)g + (chunks > 1 ? halo * (double)(chunks - 1) / chunks : 0.0);
@@ -272,6 +274,46 @@ int seam_rows_capacity(int64_t max_rows) {
   return cap + 64 > INT32_MAX / 8 ? -1 : (int)cap;
 }
 
+// What a strip's row of a sweep kernel costs, in cycles of one SM sub-partition:
+// of a warp that has it to itself, and of each of several warps that share it.
+// The second is the rate of a full GPU (FP16 pairs 17.8 Tcell/s at 48 cells per
+// lane, FP32 12.9 at 48, MIXED 13.9 at 64), the first comes from one-read batches.
+struct RowCost {
+  int S;
+  double alone, shared;
+};
+constexpr RowCost kRowCost[3][3] = {{{32, 250, 156}, {48, 265, 217}, {0, 0, 0}},
+                                    {{16, 150, 65}, {32, 230, 111}, {48, 290, 152}},
+                                    {{32, 260, 115}, {48, 320, 148}, {64, 360, 184}}};
+
+// Estimated time (in cycles) of a NO_REF_DEL sweep of `items` equal work items
+// on `teams` CTAs of k warps: an item is `work` strips' worth of rows in
+// `strips` strips.  The warps of a CTA sweep strips as a pipeline, each one
+// 32-row window behind its left neighbour, and share the SM's schedulers; both
+// limits are real at once near the middle, so they add in squares (within 10 %
+// of 270 measured shapes of eight batches, FP32 and MIXED cells).
+double sweep_estimate(const RowCost &c, int64_t items, double work, double strips, double rows, int k, int64_t teams,
+                      int sms) {
+  const double per_team = std::ceil((double)items / (double)teams) * work;
+  const double alone = c.alone * (rows * std::max(1.0, per_team / k) + kWarp * (std::min(strips, (double)k) - 1.0));
+  const double ctas_per_sm = (double)teams / sms;
+  const double used = std::min(1.0, (double)items / (double)teams);
+  const double shared = per_team * rows * c.shared / 4.0 * std::max(1.0, ctas_per_sm * used);
+  return std::sqrt(alone * alone + shared * shared);
+}
+
+// Warps of a CTA (the team that sweeps an item's strips) when nothing fixes
+// them: all that fit on an SM, which leaves the fewest idle at the end of a
+// batch (5 Mb, 96 uneven reads: 246 ms, 291 with 2-warp teams).  4-warp teams
+// for reads too short to keep a long pipeline full (176 reads of 369 samples:
+// 459 against 490 us), and for FP16 batches of many items, where nothing is
+// left of the first reason and the shorter pipeline waits less (1.3 %).
+int default_team(int precision, int full, double mean_rows, int64_t items, int sms) {
+  if (mean_rows < 640) return 4;
+  if (precision == 0 && items >= (int64_t)8 * sms * (full / 4)) return 4;
+  return full;
+}
+
 // Launch shape of a sweep: user-fixed fields win, then an autotuned entry for
 // this (precision, batch size, read length) bucket, then the defaults; the
 // chunk width comes from the analytic model (times the tuned factor).
@@ -283,21 +325,50 @@ Shape pick_shape(dtwx_handle *h, int precision, int64_t n_tasks, double mean_row
   auto t = h->tuned.find(std::make_tuple(precision, log2_bucket((double)n_tasks), log2_bucket(mean_rows)));
   const bool use_t = t != h->tuned.end();
   // defaults measured on the 1 Mb / 2,048-read batch: 48 cells per lane (64 for
-  // MIXED, whose reference takes half the registers) in 4-warp CTAs; the REF_DEL
-  // kernels default to 32 cells per lane (FP32 cells also have a 16-cell instance)
+  // MIXED, whose reference takes half the registers); the REF_DEL kernels
+  // default to 32 cells per lane (FP32 cells also have a 16-cell instance)
   const bool rd = h->cfg.recurrence == DTWX_REF_DEL;
   const int def_S = rd ? 32 : (precision == 2 ? 64 : 48);
   s.S = o.S ? o.S : (f.S ? f.S : (use_t ? t->second.S : def_S));
   const int strands = precision == 0 ? 1 : (h->cfg.strand_mode == DTWX_STRANDS_CONCAT ? 1 : 2);
+  const int64_t nt = std::max<int64_t>(n_tasks, 1) * strands;
   // warps per CTA: while tuning the candidate's (0 = the default below), else
   // user-fixed, then autotuned, then the default
   s.warps = o.S ? o.warps : (f.warps ? f.warps : (use_t ? t->second.warps : 0));
+  const bool auto_warps = s.warps <= 0 && !rd;
   if (s.warps <= 0) s.warps = rd ? refdel_spread_warps(precision, n_tasks * strands, h->sms) : 4;
   s.warps = std::min(s.warps, max_warps_per_cta(precision, rd));
   if (use_t && !f.G) g_scale = t->second.g_scale;
   if (o.S) g_scale = o.items > 0 ? o.items / 1000.0 : 1.0;  // candidate factor (per mille) while tuning
-  int occ = sdtw_ctas_per_sm(precision, s.S, s.warps, rd);
-  if (occ <= 0) occ = 1;
+  int occ = std::max(1, sdtw_ctas_per_sm(precision, s.S, s.warps, rd));
+  if (!rd && precision != 0 && !o.S && !use_t && !f.G && auto_warps) {
+    // FP32 path cost: any strip width and any chunks give the same bits, so the
+    // estimate picks both
+    double best = 1e300;
+    for (const RowCost &c : kRowCost[precision]) {
+      if (f.S && c.S != f.S) continue;
+      const int full = 4 * sdtw_ctas_per_sm(precision, c.S, 4, rd);
+      if (full <= 0 || sdtw_ctas_per_sm(precision, c.S, full, rd) < 1) continue;
+      const int k = default_team(precision, full, mean_rows, 0, h->sms);
+      const int64_t teams = (int64_t)h->sms * full / k;
+      const int W = kWarp * c.S;
+      const int64_t strips = (h->m_cols + W - 1) / W;
+      int64_t chunks = 0;
+      for (int64_t g = 1; g <= strips; g = chunks > 1 ? (strips + chunks - 2) / (chunks - 1) : g + 1) {
+        chunks = (strips + g - 1) / g;
+        const double halo = chunks > 1 ? (mean_rows + W) / (2.0 * W) * (double)(chunks - 1) / (double)chunks : 0.0;
+        const double nh = chunks > 1 ? std::ceil(mean_rows / W) : 0.0;
+        const double e = sweep_estimate(c, nt * chunks, (double)g + halo, (double)g + nh, mean_rows, k, teams, h->sms);
+        if (e < best * 0.999) {
+          best = e;
+          s.S = c.S;
+          s.G = (int)g;
+          s.warps = k;
+          occ = full / k;
+        }
+      }
+    }
+  }
   const int W = kWarp * s.S;
   const int64_t strips = (h->m_cols + W - 1) / W;
   const int64_t total_warps = (int64_t)h->sms * occ * s.warps;
@@ -305,9 +376,10 @@ Shape pick_shape(dtwx_handle *h, int precision, int64_t n_tasks, double mean_row
     s.G = (int)strips;  // REF_DEL: one chunk per task (a horizontal run crosses any chunk edge)
   } else if (f.G && !o.S) {
     s.G = f.G;
-  } else {
-    // FP16 pairs: narrow chunks get the narrow-halo instance, so price their halo that way
-    const int64_t nt = std::max<int64_t>(n_tasks, 1) * strands;
+  } else if (s.G == 0) {
+    // FP16 pairs: the frames (and with them the rounding) depend on the chunk
+    // edges, so the chunks of a batch stay what this model gives.  Narrow chunks
+    // get the narrow-halo instance, so their halo is priced that way
     int g0 = choose_chunk_strips(strips, nt, mean_rows, W, precision == 0 ? kWarp * kNarrowHaloCells : W,
                                  total_warps);
     if (precision == 0 && g0 > kNarrowHaloMaxStrips) g0 = choose_chunk_strips(strips, nt, mean_rows, W, W, total_warps);
@@ -316,22 +388,25 @@ Shape pick_shape(dtwx_handle *h, int precision, int64_t n_tasks, double mean_row
   if (s.G > strips) s.G = (int)strips;
   const int64_t chunks = (strips + s.G - 1) / s.G;
   s.nh = precision == 0 && !rd && chunks > 1 && s.G <= kNarrowHaloMaxStrips && s.S % kNarrowHaloCells == 0;
-  const int64_t items = n_tasks * chunks * strands;
-  // FP16 pairs, default shape, a batch of several waves: the SM's warps in one
-  // CTA instead of occ 4-warp CTAs (the same warps per SM, so the same chunks
-  // and bits).  Measured on the 2,048-read / 1 Mb batch at 48 cells per lane:
-  // 487 against 501 ms; equal on the 8,192-read / 5 Mb one.  Single-wave
-  // batches (serving) keep 4-warp CTAs, which leave room for the next batch.
-  if (!rd && precision == 0 && !o.S && !f.warps && !use_t && items >= 2 * total_warps && occ > 1) {
+  s.items = n_tasks * chunks * strands;
+  if (auto_warps && (precision == 0 || s.warps == 4)) {
     const int full = occ * s.warps;
-    if (sdtw_ctas_per_sm(precision, s.S, full, false) == 1) {
-      s.warps = full;
-      occ = 1;
+    const int k = default_team(precision, full, mean_rows, s.items, h->sms);
+    if (k != s.warps && sdtw_ctas_per_sm(precision, s.S, k, false) >= 1) {
+      s.warps = k;
+      occ = full / k;
     }
   }
-  s.items = items;
-  const int64_t want = (items + s.warps - 1) / s.warps;
-  s.grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)h->sms * occ, want));
+  if (rd) {
+    const int64_t want = (s.items + s.warps - 1) / s.warps;
+    s.grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)h->sms * occ, want));
+  } else {
+    s.grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)h->sms * occ, s.items));
+    // when every strip of the batch can run at once, deal the items out evenly:
+    // the CTAs that start first would take more than their share
+    const int64_t halo_strips = chunks > 1 ? (int64_t)std::ceil(mean_rows / (s.nh ? kWarp * kNarrowHaloCells : W)) : 0;
+    s.deal = s.items * (s.G + halo_strips) <= (int64_t)s.grid * s.warps * 3 / 2;
+  }
   return s;
 }
 
@@ -365,7 +440,14 @@ int enqueue_sweep(dtwx_handle *h, BatchCtx &c, int precision, cudaStream_t st, c
   }
   int32_t *counter = c.flags.as<int32_t>();
   int32_t *err = counter + 4;
-  CK(h, launch_reset(c.keys.as<unsigned long long>(), 2 * n_slots, counter, err, st));
+  // resumed reads: a counter per work item of the halo strips that have read their row state
+  int n_halo = 0;
+  if (state && n_tasks > 0) {
+    n_halo = (int)sh.items;
+    CK(h, c.halo_read.ensure(sizeof(int32_t) * (size_t)n_halo));
+  }
+  CK(h, launch_reset(c.keys.as<unsigned long long>(), 2 * n_slots, counter, err, c.halo_read.as<int32_t>(), n_halo,
+                     st));
   ++launches;
   if (n_tasks > 0) {
     SdtwParams p{};
@@ -377,6 +459,7 @@ int enqueue_sweep(dtwx_handle *h, BatchCtx &c, int precision, cudaStream_t st, c
     p.seam = c.seam.as<char>();
     p.counter = counter;
     p.err = err;
+    p.halo_read = n_halo ? c.halo_read.as<int32_t>() : nullptr;
     p.ref_plain = ref_for(h, precision);
     p.m = h->m_cols;
     p.m_pad = h->m_pad;
@@ -393,6 +476,7 @@ int enqueue_sweep(dtwx_handle *h, BatchCtx &c, int precision, cudaStream_t st, c
     p.ref_del = h->cfg.recurrence == DTWX_REF_DEL ? 1 : 0;
     p.state_fp16 = state_fp16(h) ? 1 : 0;
     p.narrow_halo = sh.nh ? 1 : 0;
+    p.deal = sh.deal ? 1 : 0;
     p.stall_item = h->stall_item;
     p.spin_limit = h->stall_spin;
     h->stall_item = 0;
@@ -663,7 +747,9 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
       p.n_items = p.n_chunks * (precision != 0 ? p.strands : 1);
       p.ref_layout = 1;
       p.narrow_halo = sh.nh ? 1 : 0;
-      const int ii = inst_index(precision, sh.S);
+      p.deal = sh.deal ? 1 : 0;
+    p.deal = sh.deal ? 1 : 0;
+        const int ii = inst_index(precision, sh.S);
       p.use_tma = h->tmap_ok[precision][ii] ? 1 : 0;
       CK(h, launch_sdtw(precision, sh.S, sh.warps, sh.grid, p, p.use_tma ? &h->tmap[precision][ii] : nullptr,
                         st));
@@ -904,6 +990,7 @@ int dtwx_destroy(dtwx_handle *h) {
     c.results.release();
     c.seam.release();
     c.flags.release();
+    c.halo_read.release();
     c.h_raw.release();
     c.h_meta.release();
     c.h_results.release();

@@ -32,6 +32,9 @@ constexpr int kNarrowHaloMaxStrips = 32;
 // microseconds.  The count does not advance while the context is switched out.
 constexpr uint32_t kSpinLimit = 1u << 18;
 
+// Shared-memory bytes of a CTA's team state (lock, abort flag, hand-out cursor).
+constexpr size_t kTeamStateBytes = 32;
+
 // Task flags.
 constexpr int32_t kTaskResume = 1;    // start from the saved row state instead of free start
 constexpr int32_t kTaskSaveState = 2; // write the final DP row to the row state
@@ -66,6 +69,8 @@ struct SdtwParams {
   char *seam;                  // per-warp scratch (seam columns + epoch offsets)
   int32_t *counter;            // work-queue ticket counter (zeroed before launch)
   int32_t *err;                // device error flags
+  int32_t *halo_read;          // per item: resumed halo strips that have read their row state (zeroed
+                               // before launch); NULL when no task both resumes and saves
   const void *ref_plain;       // reference in global memory (used when TMA is off)
   int64_t m;                   // valid columns per strand
   int64_t m_pad;               // padded columns (multiple of the strip width)
@@ -83,6 +88,7 @@ struct SdtwParams {
   int32_t state_fp16;          // FP16 cells: row state as half2 cells (m_pad) then one float2
                                // frame offset per 512-column group (m_pad / 512)
   int32_t narrow_halo;         // FP16 pairs: launch the instance with kNarrowHaloCells-wide halo strips
+  int32_t deal;                // 1: CTA b takes items b, b + grid, ...; 0: the next ticket of `counter`
   uint32_t spin_limit;         // polls before a bounded wait gives up; 0 = kSpinLimit
   int32_t stall_item;          // test hook: 1 + the queue ticket whose first reference-strip copy
                                // is not issued, so that its warp's bounded wait runs out; 0 = none
@@ -172,10 +178,10 @@ cudaError_t launch_finalize(const unsigned long long *keys, const int32_t *n_sam
                             int n_reads, int concat, int64_t m_fwd, float threshold,
                             const int32_t *err, void *d_results, cudaStream_t s);
 
-// Reset keys to the empty value, the work counter and the device error word
-// (either may be NULL) to zero.
-cudaError_t launch_reset(unsigned long long *keys, int n_keys, int32_t *counter, int32_t *err,
-                         cudaStream_t s);
+// Reset keys to the empty value, the work counter, the device error word and
+// the halo counters (each may be NULL) to zero.
+cudaError_t launch_reset(unsigned long long *keys, int n_keys, int32_t *counter, int32_t *err, int32_t *halo_read,
+                         int n_halo, cudaStream_t s);
 
 // Record the message dtwx_last_error(NULL) reports (calls made without a handle).
 void set_create_error(const char *msg);

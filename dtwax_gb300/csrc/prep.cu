@@ -253,17 +253,19 @@ cudaError_t launch_normalize(const void *src, int is_i16, const int64_t *src_off
 
 // ---------------------------------------------------------------- reset / finalize
 
-__global__ void reset_kernel(unsigned long long *keys, int n_keys, int32_t *counter, int32_t *err) {
+__global__ void reset_kernel(unsigned long long *keys, int n_keys, int32_t *counter, int32_t *err,
+                             int32_t *halo_read, int n_halo) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n_keys) keys[i] = ~0ull;
+  if (i < n_halo) halo_read[i] = 0;
   if (i == 0 && counter) *counter = 0;
   if (i == 0 && err) *err = 0;
 }
 
-cudaError_t launch_reset(unsigned long long *keys, int n_keys, int32_t *counter, int32_t *err,
-                         cudaStream_t s) {
-  const int n = n_keys > 1 ? n_keys : 1;
-  reset_kernel<<<(n + kBlock - 1) / kBlock, kBlock, 0, s>>>(keys, n_keys, counter, err);
+cudaError_t launch_reset(unsigned long long *keys, int n_keys, int32_t *counter, int32_t *err, int32_t *halo_read,
+                         int n_halo, cudaStream_t s) {
+  const int most = n_keys > n_halo ? n_keys : n_halo, n = most > 1 ? most : 1;
+  reset_kernel<<<(n + kBlock - 1) / kBlock, kBlock, 0, s>>>(keys, n_keys, counter, err, halo_read, n_halo);
   return cudaGetLastError();
 }
 

@@ -212,18 +212,43 @@ __device__ __forceinline__ void st_shared_if(uint32_t addr, uint32_t v, uint32_t
                : "memory");
 }
 
-// Drop one 128-byte L2 line without writing it back (PTX discard.global.L2,
-// sm_80 and later), issued by the lanes whose pred is set.  The contents of
-// the line become undefined; used on seam windows that have been consumed.
-__device__ __forceinline__ void discard_l2_if(const void *line, uint32_t pred) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p discard.global.L2 [%0], 128;\n\t}" ::"l"(line),
-               "r"(pred));
-}
-
 __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
   return v;
+}
+
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+// N = 2 or 4 consecutive 32-bit words from shared memory.
+template <int N>
+__device__ __forceinline__ void ld_shared_words(uint32_t addr, uint32_t (&v)[N]) {
+  static_assert(N == 2 || N == 4, "one vector load");
+  if constexpr (N == 2)
+    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(addr) : "memory");
+  else
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(addr)
+                 : "memory");
+}
+
+__device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ void st_shared_v4_if(uint32_t addr, uint4 v, uint32_t pred) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t@p st.shared.v4.b32 [%0], {%1, %2, %3, %4};\n\t}" ::"r"(addr),
+      "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(pred)
+      : "memory");
 }
 
 // Byte offset of logical byte b of a tile written by TMA with 128-byte
@@ -288,6 +313,19 @@ __device__ __forceinline__ uint32_t cell_bits(typename Pol<PREC>::V v) {
   return u;
 }
 
+// Bit image of a query sample as the policy's cells take it, and back.
+template <int PREC>
+__device__ __forceinline__ uint32_t qw_bits(float q) {
+  const typename Pol<PREC>::QW w = Pol<PREC>::qw(q);
+  uint32_t u;
+  memcpy(&u, &w, 4);
+  return u;
+}
+template <int PREC>
+__device__ __forceinline__ typename Pol<PREC>::QW qw_from(uint32_t u) {
+  return bits_as<typename Pol<PREC>::QW>(u);
+}
+
 // All-ones on lane 0, zero elsewhere, from an opaque move: the optimiser cannot
 // see which lanes hold which value, so it cannot split the row loop into a
 // lane-0 copy and a lanes-1..31 copy (which halves the active lanes of every
@@ -309,6 +347,20 @@ __device__ __forceinline__ void sweep_row(typename Pol<PREC>::V (&D)[S], const t
   using P = Pol<PREC>;
   const typename P::V up = P::shfl_up(D[S - 1]);
   const typename P::V left = P::from_bits((cell_bits<PREC>(up) & ~m0) | (cell_bits<PREC>(seam) & m0));
+  if constexpr (PREC == 1) {
+    // two columns per packed FP32 operation: the cell's three issue slots become
+    // two, with the bits of the scalar operations
+    const float2 nq = make_float2(-qq, -qq);
+#pragma unroll
+    for (int k = S - 2; k >= 0; k -= 2) {
+      const float2 m = make_float2(fminf(D[k], k > 0 ? D[k - 1] : left), fminf(D[k + 1], D[k]));
+      const float2 d = __fadd2_rn(make_float2(R[k], R[k + 1]), nq);
+      const float2 c = __ffma2_rn(d, d, m);
+      D[k] = c.x;
+      D[k + 1] = c.y;
+    }
+    return;
+  }
 #pragma unroll
   for (int k = S - 1; k >= 1; --k) D[k] = P::cell(R[k], qq, D[k], D[k - 1]);
   D[0] = P::cell(R[0], qq, D[0], left);
@@ -348,6 +400,442 @@ __device__ __forceinline__ void row(typename Pol<PREC>::V (&D)[S],
 template <int S, int PREC>
 constexpr int sdtw_reg_cap() { return S + S * Pol<PREC>::RB / 4 + 40 <= 128 ? 128 : 168; }
 
+// ---------------------------------------------------------------- the team
+// The warps of a CTA sweep the strips of an item as a pipeline.  A strip's row
+// i needs only the left neighbour's row i - 1, so strip s + 1 runs one
+// 32-row window behind strip s on another warp, through the same seam columns
+// that used to pass from one strip to the next inside one warp: the cells, the
+// frames and the order of every operation on them stay as they are.
+//
+// Strips are handed out in sequence (all of an item's, then the next item's),
+// so a strip's left neighbour was always handed out before it, and no warp
+// waits for work that has not begun.  Strip `seq` of a CTA writes its seam
+// column into buffer seq % (2 * warps); prog[] of that buffer holds the
+// sequence number and how many windows of it are complete.
+struct TeamState {
+  uint32_t lock;
+  uint32_t abort;  // a wait of this CTA gave up: every warp leaves
+  int32_t item;    // item being handed out
+  int32_t next;    // its next strip
+  int32_t total;   // its strips
+  uint32_t seq;    // strips handed out so far
+  int32_t dealt;   // items begun (p.deal)
+  uint32_t pad;
+};
+static_assert(sizeof(TeamState) == kTeamStateBytes, "shared-memory layout of the team");
+
+constexpr uint32_t kWindowsDone = 0xffffffffu;  // prog[]: every row of the strip is complete
+
+__device__ __forceinline__ uint32_t ld_shared_volatile(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void st_shared_volatile(uint32_t addr, uint32_t v) {
+  asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+// Bounded wait until prog word `addr` reaches `target`; false when the limit
+// is reached or another warp of the CTA gave up.  The limit grows with the
+// rows of a strip (the longest wait that can be in order is a strip's sweep);
+// for a 2,000-row read it ends after a fraction of a second.
+__device__ __forceinline__ bool team_wait(uint32_t addr, uint64_t target, uint32_t abort_addr, int rows) {
+  const uint32_t limit = (1u << 22) + 256u * (uint32_t)min(rows, 1 << 23);
+  for (uint32_t it = 0; it < limit; ++it) {
+    uint64_t v;
+    asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
+    if (__all_sync(FULL_MASK, v >= target)) {
+      __threadfence_block();
+      return true;
+    }
+    if (__any_sync(FULL_MASK, ld_shared_volatile(abort_addr) != 0)) return false;
+    __nanosleep(40);
+  }
+  return false;
+}
+
+// One look at a prog word, without waiting.
+__device__ __forceinline__ bool team_ready(uint32_t addr, uint64_t target) {
+  uint64_t v;
+  asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
+  const bool ready = __all_sync(FULL_MASK, v >= target);
+  __threadfence_block();
+  return ready;
+}
+
+// Windows 0 .. windows-1 of the strip are complete (or all of it): the seam
+// values and offsets every lane stored before are visible to the CTA's other
+// warps first.
+__device__ __forceinline__ void team_publish(uint32_t addr, uint32_t seq, uint32_t windows) {
+  __threadfence_block();
+  __syncwarp();
+  const uint64_t v = ((uint64_t)(seq + 1) << 32) | windows;
+  asm volatile("st.volatile.shared.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+}
+
+// The item's geometry: its columns [a, b), where its halo starts and its strips.
+struct Item {
+  int64_t a, b, x0;
+  int nh, nstrips;
+};
+template <int W, int WH>
+__device__ __forceinline__ Item item_geometry(const SdtwParams &p, int chunk, int n) {
+  Item g;
+  const int64_t C = (int64_t)p.chunk_strips * W;
+  g.a = (int64_t)chunk * C;
+  g.b = min(g.a + C, p.m);
+  g.x0 = g.a;
+  if (chunk > 0) {
+    const int64_t halo = ((int64_t)n + WH - 1) / WH * WH;
+    g.x0 = g.a - halo > 0 ? g.a - halo : 0;
+  }
+  g.nh = (int)((g.a - g.x0) / WH);
+  g.nstrips = g.nh + (int)((g.b - g.a + W - 1) / W);
+  return g;
+}
+
+// ---------------------------------------------------------------- row state
+
+// Row "-1" of a resumed strip's columns [c0, c0 + SC) of this lane, and the
+// frame offset (FP16 cells: the strip's minimum).
+template <int SC, int PREC, bool ST16>
+__device__ __forceinline__ void load_row_state(typename Pol<PREC>::V (&D)[SC], float2 &O, const float *plane0,
+                                               int64_t m_pad, int strand, int64_t c0) {
+  if constexpr (PREC == 0) {
+    float mx = __int_as_float(0x7f800000), my = mx;
+    if constexpr (ST16) {
+      // FP16 row state: half2 cells relative to the offset of their 512-column
+      // group (the saving strip's frame); re-based onto this strip's minimum
+      const uint4 *hc = reinterpret_cast<const uint4 *>(reinterpret_cast<const __half2 *>(plane0) + c0);
+      const float2 *og = reinterpret_cast<const float2 *>(plane0 + m_pad);
+#pragma unroll
+      for (int k = 0; k < SC / 4; ++k) {
+        const uint4 u = hc[k];
+        D[4 * k] = bits_as<__half2>(u.x);
+        D[4 * k + 1] = bits_as<__half2>(u.y);
+        D[4 * k + 2] = bits_as<__half2>(u.z);
+        D[4 * k + 3] = bits_as<__half2>(u.w);
+      }
+#pragma unroll
+      for (int k = 0; k < SC; ++k) {
+        const float2 o = og[(c0 + k) >> 9];
+        const float2 v = __half22float2(D[k]);
+        mx = fminf(mx, v.x + o.x);
+        my = fminf(my, v.y + o.y);
+      }
+    } else {
+      // two passes over the saved planes: strip minimum first, then the cells
+      const float4 *f0 = reinterpret_cast<const float4 *>(plane0 + c0);
+      const float4 *f1 = reinterpret_cast<const float4 *>(plane0 + m_pad + c0);
+#pragma unroll
+      for (int k = 0; k < SC / 4; ++k) {
+        const float4 u = f0[k], v = f1[k];
+        mx = fminf(mx, fminf(fminf(u.x, u.y), fminf(u.z, u.w)));
+        my = fminf(my, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
+      }
+    }
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) {
+      mx = fminf(mx, __shfl_xor_sync(FULL_MASK, mx, m));
+      my = fminf(my, __shfl_xor_sync(FULL_MASK, my, m));
+    }
+    O = make_float2(mx, my);
+    if constexpr (ST16) {
+      const float2 *og = reinterpret_cast<const float2 *>(plane0 + m_pad);
+#pragma unroll
+      for (int k = 0; k < SC; ++k) {
+        const float2 o = og[(c0 + k) >> 9];
+        const float2 v = __half22float2(D[k]);
+        D[k] = __floats2half2_rn(v.x + o.x - mx, v.y + o.y - my);
+      }
+    } else {
+      const float4 *f0 = reinterpret_cast<const float4 *>(plane0 + c0);
+      const float4 *f1 = reinterpret_cast<const float4 *>(plane0 + m_pad + c0);
+#pragma unroll
+      for (int k = 0; k < SC / 4; ++k) {
+        const float4 u = f0[k], v = f1[k];
+        D[4 * k] = __floats2half2_rn(u.x - mx, v.x - my);
+        D[4 * k + 1] = __floats2half2_rn(u.y - mx, v.y - my);
+        D[4 * k + 2] = __floats2half2_rn(u.z - mx, v.z - my);
+        D[4 * k + 3] = __floats2half2_rn(u.w - mx, v.w - my);
+      }
+    }
+  } else {
+    const float4 *f = reinterpret_cast<const float4 *>(plane0 + (int64_t)strand * m_pad + c0);
+#pragma unroll
+    for (int k = 0; k < SC / 4; ++k) {
+      const float4 u = f[k];
+      D[4 * k] = u.x;
+      D[4 * k + 1] = u.y;
+      D[4 * k + 2] = u.z;
+      D[4 * k + 3] = u.w;
+    }
+  }
+}
+
+// The last row of this lane's columns, back to the read's row state.
+template <int S, int PREC, bool ST16>
+__device__ __forceinline__ void save_row_state(const typename Pol<PREC>::V (&D)[S], float2 O, float *plane0,
+                                               int64_t m_pad, int strand, int64_t c0) {
+  if constexpr (PREC == 0 && ST16) {
+    // half2 cells in this strip's frame, the frame offset once per 512-column group
+    uint4 *hc = reinterpret_cast<uint4 *>(reinterpret_cast<__half2 *>(plane0) + c0);
+#pragma unroll
+    for (int k = 0; k < S / 4; ++k)
+      hc[k] = make_uint4(cell_bits<0>(D[4 * k]), cell_bits<0>(D[4 * k + 1]), cell_bits<0>(D[4 * k + 2]),
+                         cell_bits<0>(D[4 * k + 3]));
+    float2 *og = reinterpret_cast<float2 *>(plane0 + m_pad);
+    og[c0 >> 9] = O;  // every lane of the strip stores the same value
+    og[(c0 + S - 1) >> 9] = O;
+  } else if constexpr (PREC == 0) {
+    float4 *f0 = reinterpret_cast<float4 *>(plane0 + c0);
+    float4 *f1 = reinterpret_cast<float4 *>(plane0 + m_pad + c0);
+#pragma unroll
+    for (int k = 0; k < S / 4; ++k) {
+      const float2 v0 = __half22float2(D[4 * k]), v1 = __half22float2(D[4 * k + 1]);
+      const float2 v2 = __half22float2(D[4 * k + 2]), v3 = __half22float2(D[4 * k + 3]);
+      f0[k] = make_float4(v0.x + O.x, v1.x + O.x, v2.x + O.x, v3.x + O.x);
+      f1[k] = make_float4(v0.y + O.y, v1.y + O.y, v2.y + O.y, v3.y + O.y);
+    }
+  } else {
+    float4 *f = reinterpret_cast<float4 *>(plane0 + (int64_t)strand * m_pad + c0);
+#pragma unroll
+    for (int k = 0; k < S / 4; ++k) f[k] = make_float4(D[4 * k], D[4 * k + 1], D[4 * k + 2], D[4 * k + 3]);
+  }
+}
+
+// Wait until the resumed halos that start from the saved row of columns
+// [x, x + W) have read it: the halos of the chunks to the right of this one
+// that reach column x.  Those chunks were handed out before this one and their
+// halo strips depend on nothing of it.  Bounded like team_wait.
+template <int W, int WH>
+__device__ __forceinline__ bool wait_halo_readers(const SdtwParams &p, const Item &g, int64_t x, int item, int chunk,
+                                                  int n, uint32_t abort_addr) {
+  for (int c = chunk + 1; c < p.n_chunks; ++c) {
+    const Item h = item_geometry<W, WH>(p, c, n);
+    if (h.x0 >= x + W) break;
+    const uint32_t limit = (1u << 22) + 256u * (uint32_t)min(n, 1 << 23);
+    bool done = false;
+    for (uint32_t it = 0; it < limit && !done; ++it) {
+      int32_t v;
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(&p.halo_read[item - (c - chunk)]) : "memory");
+      done = __all_sync(FULL_MASK, v >= h.nh);
+      if (!done) {
+        if (__any_sync(FULL_MASK, ld_shared_volatile(abort_addr) != 0)) return false;
+        __nanosleep(100);
+      }
+    }
+    if (!done) return false;
+  }
+  return true;
+}
+
+// ---------------------------------------------------------------- one strip
+
+// What a strip's sweep is given besides its columns (all warp-uniform).
+struct Strip {
+  int64_t x;         // first column
+  int rows;          // rows to sweep: n, or fewer in a halo strip
+  int n;             // rows of the read
+  int strand;
+  bool first;        // leftmost strip of its item
+  bool resume;
+  const float *q;
+  const float *st_plane0;
+  uint32_t seq;      // its place in the CTA's sequence
+  char *in_b, *out_b;          // seam columns of the left neighbour and of this strip
+  uint32_t prog_in, prog_out;  // their progress words
+};
+
+// Sweeps SC cells per lane through the strip's rows; the last row is left in
+// D, its frame in O.  False when a wait gave up.
+template <int SC, int PREC, bool ST16, typename OnLoaded>
+__device__ __forceinline__ bool sweep_strip(const SdtwParams &p, const Strip &st, typename Pol<PREC>::V (&D)[SC],
+                                            float2 &O, int lane, uint32_t m0, uint32_t is31, uint32_t wb,
+                                            const unsigned char *slot, uint64_t *bar, uint32_t &phase,
+                                            uint32_t spin_limit, uint32_t abort_addr, OnLoaded on_loaded) {
+  using P = Pol<PREC>;
+  using V = typename P::V;
+  using RV = typename P::RV;
+  constexpr int RB = P::RB;           // reference bytes per column
+  constexpr int NW = SC * RB / 4;     // reference words per lane
+  constexpr int K = kRescaleRows;
+  // rows per group of the window loop, and how their seam cells leave it, by
+  // what the instruction schedule measured (64 strips of one read per item,
+  // Tcell/s): FP16 pairs, 4 rows and one 16-byte store 17.8, a store per row
+  // 15.2, 2 rows 15.5; FP32, 4 rows and a store per row 12.9, one 16-byte
+  // store 12.7, 2 rows 12.5; MIXED, 2 rows and a store per row 13.9, 4 rows 13.6
+  constexpr int kRows = PREC == 2 ? 2 : 4;
+  const int n = st.n, rows = st.rows;
+  const bool first = st.first;
+  const float *q = st.q;
+  const int64_t off_pos = seam_offsets_pos(4, p.max_rows);
+  const V *seam_in = reinterpret_cast<const V *>(st.in_b);
+  const float2 *off_in = reinterpret_cast<const float2 *>(st.in_b + off_pos);
+  V *seam_out = reinterpret_cast<V *>(st.out_b);
+  float2 *off_out = reinterpret_cast<float2 *>(st.out_b + off_pos);
+
+  // -- initial row ("row -1"): zeros (free start) or the saved row state
+  O = make_float2(0.f, 0.f);  // FP16 frame offsets (fwd, rev)
+  if (st.resume) {
+    load_row_state<SC, PREC, ST16>(D, O, st.st_plane0, p.m_pad, st.strand, st.x + (int64_t)lane * SC);
+    on_loaded();
+  } else {
+#pragma unroll
+    for (int k = 0; k < SC; ++k) D[k] = P::zero();
+  }
+
+  // -- reference strip into registers (after the row state: fewer live registers)
+  RV R[NW];
+  // column offset of this item's strand in a planar reference (FP32 planes, or MIXED FP16 planes)
+  const int64_t ref_plane = (PREC == 2 || (PREC == 1 && p.ref_layout == 1)) ? (int64_t)st.strand * p.m_pad : 0;
+  if (p.use_tma) {
+    // every lane waits (acquire of the TMA bytes); the give-up decision is warp-uniform
+    if (!__all_sync(FULL_MASK, mbar_wait(bar, phase, spin_limit))) return false;
+    phase ^= 1u;
+    regs_from_smem<NW, RV>(slot, lane, R);
+    __syncwarp();
+  } else if constexpr (PREC == 1) {
+    if (p.ref_layout == 0)
+      regs_from_pairs<SC>(reinterpret_cast<const float2 *>(p.ref_plain), st.x, lane, st.strand, R);
+    else
+      regs_from_global<NW, RV>(reinterpret_cast<const float *>(p.ref_plain) + ref_plane + st.x, lane, R);
+  } else if constexpr (PREC == 2) {
+    regs_from_global<NW, RV>(reinterpret_cast<const __half *>(p.ref_plain) + ref_plane + st.x, lane, R);
+  } else {
+    regs_from_global<NW, RV>(reinterpret_cast<const __half2 *>(p.ref_plain) + st.x, lane, R);
+  }
+
+  // uniform stores (every lane writes the same value): no lane-dependent branch
+  seam_out[0] = P::shfl(D[SC - 1], 31);
+  if constexpr (PREC == 0) off_out[0] = O;
+
+  // the left neighbour's first window: seam rows -1 .. 31, offsets 0 and 1
+  const uint64_t tag_in = (uint64_t)st.seq << 32;
+  if (!first && !team_wait(st.prog_in, tag_in | 1u, abort_addr, n)) return false;
+
+  // -- row sweep, 32 rows per window.  The window's query samples, its incoming
+  // seam values (already re-based into this strip's frame; delta changes only
+  // at a rescale, which ends a window) and its outgoing ones pass through three
+  // 128-byte shared buffers: four rows take one 16-byte broadcast load of each
+  // and one 16-byte store by lane 31, where a shuffle per row and value cost
+  // four times as many issue slots.
+  const V vinf = P::inf();
+  uint32_t qb = qw_bits<PREC>(lane < n ? q[lane] : 0.f);
+  V swin = (!first && lane < rows) ? seam_in[lane] : vinf;
+  if constexpr (PREC == 0) {
+    // re-base by the offset of the left strip's frame relative to this strip's
+    const float2 oi = first ? O : off_in[0];
+    swin = __hadd2(swin, __float22half2_rn(make_float2(oi.x - O.x, oi.y - O.y)));
+  }
+  V *so = seam_out + 1;  // seam value of row i goes to seam_out[i + 1]
+  uint32_t win = 0;      // windows complete
+  for (int i0 = 0; i0 < rows; i0 += kWarp) {
+    st_shared_u32(wb + 4u * (uint32_t)lane, qb);
+    st_shared_u32(wb + 128u + 4u * (uint32_t)lane, cell_bits<PREC>(swin));
+    __syncwarp();
+    // the next window's samples, and its seam values from the left neighbour's
+    // next window.  FP32 and MIXED cells fetch what is complete ahead of this
+    // window's rows; FP16 pairs fetch it all after them (the registers that
+    // would hold it cost the rows more: 17.8 against 18.2 Tcell/s)
+    const int r = i0 + kWarp + lane;
+    const bool more = !first && i0 + kWarp < rows;
+    const bool ahead = PREC != 0 && more && team_ready(st.prog_in, tag_in | (win + 2));
+    float qn = 0.f;
+    if constexpr (PREC == 2) qn = r < n ? q[r] : 0.f;
+    V sn = vinf;
+    float2 off_next = O;
+    if (ahead && r < rows) sn = seam_in[r];
+    V sout;
+    if (rows - i0 >= kWarp) {
+      if constexpr (PREC == 0) {
+#pragma unroll 1
+        for (int g = 0; g < kWarp / 4; ++g) {
+          const uint4 qv = ld_shared_v4(wb + 16u * (uint32_t)g), sv = ld_shared_v4(wb + 128u + 16u * (uint32_t)g);
+          uint4 ov;
+          row<SC, PREC>(D, R, qw_from<PREC>(qv.x), P::from_bits(sv.x), m0);
+          ov.x = cell_bits<PREC>(D[SC - 1]);
+          row<SC, PREC>(D, R, qw_from<PREC>(qv.y), P::from_bits(sv.y), m0);
+          ov.y = cell_bits<PREC>(D[SC - 1]);
+          row<SC, PREC>(D, R, qw_from<PREC>(qv.z), P::from_bits(sv.z), m0);
+          ov.z = cell_bits<PREC>(D[SC - 1]);
+          row<SC, PREC>(D, R, qw_from<PREC>(qv.w), P::from_bits(sv.w), m0);
+          ov.w = cell_bits<PREC>(D[SC - 1]);
+          st_shared_v4_if(wb + 256u + 16u * (uint32_t)g, ov, is31);
+        }
+      } else {
+#pragma unroll 1
+        for (int g = 0; g < kWarp; g += kRows) {
+          uint32_t qv[kRows], sv[kRows];
+          ld_shared_words(wb + 4u * (uint32_t)g, qv);
+          ld_shared_words(wb + 128u + 4u * (uint32_t)g, sv);
+#pragma unroll
+          for (int j = 0; j < kRows; ++j) {
+            row<SC, PREC>(D, R, qw_from<PREC>(qv[j]), P::from_bits(sv[j]), m0);
+            st_shared_if(wb + 256u + 4u * (uint32_t)(g + j), cell_bits<PREC>(D[SC - 1]), is31);
+          }
+        }
+      }
+      __syncwarp();
+      sout = P::from_bits(ld_shared_u32(wb + 256u + 4u * (uint32_t)lane));
+      if constexpr (PREC == 0) {
+        // rescale: subtract this strip's row minimum (one epoch = 32 rows)
+        // (four partial minima: a single chain of SC dependent minima would
+        // stall the warp once per window)
+        V mq[4] = {D[0], D[1], D[2], D[3]};
+#pragma unroll
+        for (int k = 4; k < SC; ++k) mq[k & 3] = __hmin2(mq[k & 3], D[k]);
+        V mn = __hmin2(__hmin2(mq[0], mq[1]), __hmin2(mq[2], mq[3]));
+#pragma unroll
+        for (int m = 16; m >= 1; m >>= 1) mn = __hmin2(mn, P::shfl_xor(mn, m));
+#pragma unroll
+        for (int k = 0; k < SC; ++k) D[k] = __hsub2(D[k], mn);
+        const float2 mf = __half22float2(mn);
+        O.x += mf.x;
+        O.y += mf.y;
+        const int e = (i0 + kWarp) / K;
+        off_out[e] = O;  // warp-uniform value, stored by every lane
+        sout = P::sel(lane == kWarp - 1, D[SC - 1], sout);  // the seam leaves in the new frame
+      }
+      so[lane] = sout;
+    } else {
+      const int cnt = rows - i0;
+      for (int il = 0; il < cnt; ++il) {
+        row<SC, PREC>(D, R, qw_from<PREC>(ld_shared_u32(wb + 4u * (uint32_t)il)),
+                      P::from_bits(ld_shared_u32(wb + 128u + 4u * (uint32_t)il)), m0);
+        st_shared_if(wb + 256u + 4u * (uint32_t)il, cell_bits<PREC>(D[SC - 1]), is31);
+      }
+      __syncwarp();
+      // lanes >= cnt write +inf into the buffer's 32-entry slack past the rows
+      so[lane] = lane < cnt ? P::from_bits(ld_shared_u32(wb + 256u + 4u * (uint32_t)lane)) : vinf;
+    }
+    so += kWarp;
+    ++win;
+    team_publish(st.prog_out, st.seq, win);
+    if (more && !ahead) {
+      if (!team_wait(st.prog_in, tag_in | (win + 1), abort_addr, n)) return false;
+      if (r < rows) sn = seam_in[r];
+      if constexpr (PREC == 0) off_next = off_in[win];
+    }
+    if constexpr (PREC != 2) qn = r < n ? q[r] : 0.f;
+    qb = qw_bits<PREC>(qn);
+    swin = sn;
+    if constexpr (PREC == 0) {
+      if (!first) swin = __hadd2(swin, __float22half2_rn(make_float2(off_next.x - O.x, off_next.y - O.y)));
+    }
+  }
+  if (rows < n) {
+    // rows this halo strip skipped can no longer reach column a: keep them
+    // inert (whole 32-entry groups; the buffers have 32 entries of slack)
+    for (int rr = rows + 1; rr <= n; rr += kWarp) seam_out[rr + lane] = vinf;
+    if constexpr (PREC == 0) {
+      for (int e = rows / K + 1; e <= n / K; e += kWarp) off_out[e + lane] = O;
+    }
+  }
+  return true;
+}
+
 // The NO_REF_DEL sweep.  (The REF_DEL recurrence runs the anti-diagonal
 // kernels of refdel.cu.)
 // ST16: FP16 cells whose serving row state is FP16 (p.state_fp16); a separate
@@ -358,14 +846,10 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
     const __grid_constant__ CUtensorMap tmap, const SdtwParams p) {
   using P = Pol<PREC>;
   using V = typename P::V;
-  using RV = typename P::RV;
   constexpr bool PAIRS = PREC == 0;           // both strands in one cell (FP16)
   constexpr int W = kWarp * S;                // columns per strip
   constexpr int RB = P::RB;                   // reference bytes per column
-  constexpr int NW = S * RB / 4;              // reference words per lane
-  constexpr int CB = 4;                       // bytes per cell
   constexpr int STRIP_BYTES = W * RB;
-  constexpr int K = kRescaleRows;
   constexpr int SH = NH ? kNarrowHaloCells : S;  // cells per lane in halo strips
   constexpr int WH = kWarp * SH;
   static_assert(S % SH == 0 && SH % 8 == 0, "halo strips must tile the chunk start");
@@ -373,11 +857,6 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
   static_assert(STRIP_BYTES % 1024 == 0, "strip tile must keep 1024-byte alignment");
   static_assert(S % 8 == 0, "row state and reference move in 16-byte groups");
   static_assert(!ST16 || PREC == 0, "the FP16 row state is built for FP16 cells");
-  // rows unrolled in the 32-row window loop, measured per cell type (C2 and
-  // the 5 Mb uneven batch): 8 gives MIXED cells +6 %; FP16 pairs are 2 %
-  // faster with 8 on 2,000-row reads but 0.6 % slower on the uneven batch,
-  // and FP32 cells do not change; 16 loses 13-17 % everywhere
-  constexpr int kRowUnroll = PREC == 2 ? 8 : 4;
 
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>(
@@ -386,32 +865,33 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
   const int warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
   const uint32_t m0 = lane0_mask(lane);
-  unsigned char *const slot0 = smem + (2 * warp) * STRIP_BYTES;  // slot s at slot0 + s*STRIP_BYTES
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * nwarps * STRIP_BYTES) + 2 * warp;
-  // The seam column leaving a strip, gathered per 32-row window and stored
-  // coalesced.  FP32 and MIXED: lane 31 stores each row's last cell into this
-  // shared buffer (measured 1.6 % / 2.9 % faster); FP16: lane l keeps row i0+l
-  // in a register, taken from lane 31 by a shuffle (2.2 % faster than the
-  // shared buffer for half2 cells).
-  constexpr bool SMEM_SEAM = PREC != 0;
-  const uint32_t sob = smem_u32(smem + 2 * nwarps * STRIP_BYTES + 16 * nwarps) + 128u * (uint32_t)warp;
+  // per warp: a reference strip tile, its mbarrier and three 128-byte windows
+  // (query samples, seam in, seam out); per CTA: the team's state and
+  // two progress words a warp
+  unsigned char *const slot = smem + warp * STRIP_BYTES;
+  uint64_t *const bar = reinterpret_cast<uint64_t *>(smem + nwarps * STRIP_BYTES) + 2 * warp;
+  const uint32_t wb = smem_u32(smem + nwarps * (STRIP_BYTES + 16)) + 384u * (uint32_t)warp;
+  unsigned char *const team_p = smem + nwarps * (STRIP_BYTES + 16 + 384);
+  const uint32_t team = smem_u32(team_p);
+  const uint32_t prog = team + kTeamStateBytes;
+  const int nbuf = 2 * nwarps;
   uint32_t is31 = lane == kWarp - 1 ? 1u : 0u;
   asm volatile("mov.b32 %0, %0;" : "+r"(is31));  // opaque to the optimiser, like lane0_mask
 
   const uint32_t is0 = m0 & 1u;  // 1 on lane 0 (opaque to the optimiser)
   if (p.use_tma) {
-    mbar_init_if(&bars[0], 1, is0);
-    mbar_init_if(&bars[1], 1, is0);
+    mbar_init_if(bar, 1, is0);
     fence_mbar_init();
   }
-  __syncwarp();
-  uint32_t phase = 0;  // bit s = parity of the next completion of slot s
+  for (int i = threadIdx.x; i < (int)kTeamStateBytes / 4 + 4 * nwarps; i += blockDim.x)
+    reinterpret_cast<uint32_t *>(team_p)[i] = 0;
+  __syncthreads();
+  uint32_t phase = 0;  // parity of the tile's next completion
 
-  const int64_t gwarp = (int64_t)blockIdx.x * nwarps + warp;
-  char *seam_base = p.seam + gwarp * p.seam_stride;
+  const uint32_t lock_a = team, abort_a = team + 4, item_a = team + 8, next_a = team + 12, total_a = team + 16,
+                 seq_a = team + 20, dealt_a = team + 24;
+  char *const seam_base = p.seam + (int64_t)blockIdx.x * nwarps * p.seam_stride;
   const int64_t seam_half = p.seam_stride / 2;
-  const int64_t off_pos = seam_offsets_pos(CB, p.max_rows);
-  const int64_t C = (int64_t)p.chunk_strips * W;
   // FP32 and MIXED split each (task, chunk) into one work item per strand
   const int nstr = !PAIRS ? (p.strands > 0 ? p.strands : 2) : 1;
   const int per_task = p.n_chunks * nstr;
@@ -419,585 +899,176 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
   const uint32_t spin_limit = p.spin_limit ? p.spin_limit : kSpinLimit;
 
   for (;;) {
-    const int item = __shfl_sync(FULL_MASK, ticket_if(p.counter, is0), 0);
+    // -- the next strip of the CTA's sequence, under the team's lock.  Every
+    // lane runs the same instructions (only the atomics are lane 0's).
+    bool held = false;
+    for (uint32_t it = 0; it < (1u << 22) && !held; ++it) {
+      held = __shfl_sync(FULL_MASK, lock_if(lock_a, is0), 0) == 0;
+      if (!held) __nanosleep(20);
+    }
+    __threadfence_block();
+    if (!held || __any_sync(FULL_MASK, ld_shared_volatile(abort_a) != 0)) {
+      atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
+      st_shared_volatile(abort_a, 1);
+      if (held) st_shared_volatile(lock_a, 0);
+      return;
+    }
+    int item = (int)ld_shared_volatile(item_a);
+    int s = (int)ld_shared_volatile(next_a);
+    int total = (int)ld_shared_volatile(total_a);
+    const uint32_t seq = ld_shared_volatile(seq_a);
+    while (s >= total && item < n_items) {
+      if (p.deal) {
+        const uint32_t dealt = ld_shared_volatile(dealt_a);
+        item = (int)(blockIdx.x + dealt * gridDim.x);
+        __syncwarp();
+        st_shared_volatile(dealt_a, dealt + 1);
+        __syncwarp();
+      } else {
+        item = __shfl_sync(FULL_MASK, ticket_if(p.counter, is0), 0);
+      }
+      if (item >= n_items) break;
+      const int tr = item / per_task;
+      const int n = p.tasks[p.order ? p.order[tr] : tr].n;
+      if (n <= 0 || n > p.max_rows) {
+        if (n > p.max_rows) atomicOr(p.err, kErrBadTask);  // every lane: same bit
+        continue;
+      }
+      const int rem = item - tr * per_task;
+      const int chunk = p.n_chunks - 1 - (!PAIRS ? rem % p.n_chunks : rem);
+      s = 0;
+      total = item_geometry<W, WH>(p, chunk, n).nstrips;
+    }
+    __syncwarp();
+    st_shared_volatile(item_a, (uint32_t)(item < n_items ? item : (int)n_items));
+    st_shared_volatile(next_a, (uint32_t)(s + 1));
+    st_shared_volatile(total_a, (uint32_t)total);
+    st_shared_volatile(seq_a, seq + 1);
+    __threadfence_block();
+    __syncwarp();
+    st_shared_volatile(lock_a, 0);
     if (item >= n_items) break;
+
     const int tr = item / per_task;
     const int rem = item - tr * per_task;
+    // Chunks go from right to left: a resumed chunk's halo reads the saved row
+    // of the columns to its left before their own chunks overwrite it.
     const int strand = !PAIRS ? rem / p.n_chunks : 0;
-    const int chunk = rem - strand * p.n_chunks;
-    const int ti = p.order ? p.order[tr] : tr;
-    const Task t = p.tasks[ti];
+    const int chunk = p.n_chunks - 1 - (rem - strand * p.n_chunks);
+    const Task t = p.tasks[p.order ? p.order[tr] : tr];
     const int n = t.n;
-    if (n <= 0 || n > p.max_rows) {
-      if (n > p.max_rows) atomicOr(p.err, kErrBadTask);  // every lane: same bit
-      continue;
-    }
-    const int64_t a = (int64_t)chunk * C;
-    const int64_t b = min(a + C, p.m);
-    // halo strips (left of a) are WH columns wide, the chunk's own strips W
-    int64_t x0 = a;
-    if (chunk > 0) {
-      const int64_t halo = ((int64_t)n + WH - 1) / WH * WH;
-      x0 = a - halo > 0 ? a - halo : 0;
-    }
-    const int nh = (int)((a - x0) / WH);
-    const int nstrips = nh + (int)((b - a + W - 1) / W);
-    // strips [0, s_main) are narrow halo strips swept by sweep_halo_strip; the
-    // loop below sweeps the rest, W wide from column xm0 (with full-width halo
-    // strips it sweeps them too)
-    const int s_main = SH != S ? nh : 0;
-    const int64_t xm0 = SH != S ? a : x0;
-    const float *q = p.query + t.q_off;
-    const bool resume = (t.flags & kTaskResume) != 0;
+    const Item g = item_geometry<W, WH>(p, chunk, n);
     const bool save = (t.flags & kTaskSaveState) != 0 && p.state != nullptr;
-    // planar row state: strand s of this read at state + state_off + s*m_pad
-    const float *st_plane0 = p.state ? p.state + t.state_off : nullptr;
-    // column offset of this item's strand in a planar reference (FP32 planes, or MIXED FP16 planes)
-    const int64_t ref_plane = (PREC == 2 || (PREC == 1 && p.ref_layout == 1)) ? (int64_t)strand * p.m_pad : 0;
+    const bool halo = s < g.nh;  // left of column a: no result
 
-    float bestx = __int_as_float(0x7f800000), besty = bestx;
-    int64_t colx = -1, coly = -1;
-
-    if (p.use_tma) {
-      // the test hook p.stall_item withholds this copy (and its arrival) for
-      // one item: the strip's wait below then runs out with no copy in flight
-      fence_proxy_async_smem();
-      tma_issue_if(slot0, &tmap, &bars[0], 0, (int)((ref_plane + x0) * RB / 128), STRIP_BYTES,
-                   is0 & (item + 1 != p.stall_item ? 1u : 0u));
-    }
-
-    // One narrow halo strip (SH cells per lane, left of column a); false if a
-    // TMA wait gave up.  The same steps as the loop below, without the
-    // result and row-state tail (a halo strip holds no output column).
-    auto sweep_halo_strip = [&](const int s) -> bool {
-      constexpr int NWH = SH * RB / 4;
-      const int64_t x = x0 + (int64_t)s * WH;
-      const bool first = (s == 0);
+    Strip st;
+    st.x = halo ? g.x0 + (int64_t)s * WH : g.a + (int64_t)(s - g.nh) * W;
+    st.n = n;
+    st.rows = n;
+    if (halo) {
       // rows that can still reach column a
-      const int64_t lim = (int64_t)n - 1 - (a - x - WH);
-      const int rows = (int)(lim < 0 ? 0 : (lim > n ? n : lim));
-
-      // -- seam buffers (ping-pong by strip parity)
-      char *in_b = seam_base + ((s + 1) & 1) * seam_half;
-      char *out_b = seam_base + (s & 1) * seam_half;
-      const V *seam_in = reinterpret_cast<const V *>(in_b);
-      const float2 *off_in = reinterpret_cast<const float2 *>(in_b + off_pos);
-      V *seam_out = reinterpret_cast<V *>(out_b);
-      float2 *off_out = reinterpret_cast<float2 *>(out_b + off_pos);
-
-      // -- initial row ("row -1"): zeros (free start) or the saved row state
-      V D[SH];
-      float2 O = make_float2(0.f, 0.f);  // FP16 frame offsets (fwd, rev)
-      if (resume) {
-        const int64_t c0 = x + (int64_t)lane * SH;
-        if constexpr (PREC == 0) {
-          if constexpr (ST16) {
-            // FP16 row state: half2 cells relative to the offset of their
-            // 512-column group (the saving strip's frame); re-based onto this
-            // strip's minimum
-            const uint4 *hc = reinterpret_cast<const uint4 *>(reinterpret_cast<const __half2 *>(st_plane0) + c0);
-            const float2 *og = reinterpret_cast<const float2 *>(st_plane0 + p.m_pad);
-  #pragma unroll
-            for (int k = 0; k < SH / 4; ++k) {
-              const uint4 u = hc[k];
-              D[4 * k] = bits_as<__half2>(u.x);
-              D[4 * k + 1] = bits_as<__half2>(u.y);
-              D[4 * k + 2] = bits_as<__half2>(u.z);
-              D[4 * k + 3] = bits_as<__half2>(u.w);
-            }
-            float mx = __int_as_float(0x7f800000), my = mx;
-  #pragma unroll
-            for (int k = 0; k < SH; ++k) {
-              const float2 o = og[(c0 + k) >> 9];
-              const float2 v = __half22float2(D[k]);
-              mx = fminf(mx, v.x + o.x);
-              my = fminf(my, v.y + o.y);
-            }
-  #pragma unroll
-            for (int m = 16; m >= 1; m >>= 1) {
-              mx = fminf(mx, __shfl_xor_sync(FULL_MASK, mx, m));
-              my = fminf(my, __shfl_xor_sync(FULL_MASK, my, m));
-            }
-            O = make_float2(mx, my);
-  #pragma unroll
-            for (int k = 0; k < SH; ++k) {
-              const float2 o = og[(c0 + k) >> 9];
-              const float2 v = __half22float2(D[k]);
-              D[k] = __floats2half2_rn(v.x + o.x - mx, v.y + o.y - my);
-            }
-          } else {
-          // two passes over the saved planes: strip minimum first, then the cells
-          const float4 *f0 = reinterpret_cast<const float4 *>(st_plane0 + c0);
-          const float4 *f1 = reinterpret_cast<const float4 *>(st_plane0 + p.m_pad + c0);
-          float mx = __int_as_float(0x7f800000), my = mx;
-  #pragma unroll
-          for (int k = 0; k < SH / 4; ++k) {
-            const float4 u = f0[k], v = f1[k];
-            mx = fminf(mx, fminf(fminf(u.x, u.y), fminf(u.z, u.w)));
-            my = fminf(my, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
-          }
-  #pragma unroll
-          for (int m = 16; m >= 1; m >>= 1) {
-            mx = fminf(mx, __shfl_xor_sync(FULL_MASK, mx, m));
-            my = fminf(my, __shfl_xor_sync(FULL_MASK, my, m));
-          }
-          O = make_float2(mx, my);
-  #pragma unroll
-          for (int k = 0; k < SH / 4; ++k) {
-            const float4 u = f0[k], v = f1[k];
-            D[4 * k] = __floats2half2_rn(u.x - mx, v.x - my);
-            D[4 * k + 1] = __floats2half2_rn(u.y - mx, v.y - my);
-            D[4 * k + 2] = __floats2half2_rn(u.z - mx, v.z - my);
-            D[4 * k + 3] = __floats2half2_rn(u.w - mx, v.w - my);
-          }
-          }
-        } else {
-          const float4 *f = reinterpret_cast<const float4 *>(st_plane0 + (int64_t)strand * p.m_pad + c0);
-  #pragma unroll
-          for (int k = 0; k < SH / 4; ++k) {
-            const float4 u = f[k];
-            D[4 * k] = u.x;
-            D[4 * k + 1] = u.y;
-            D[4 * k + 2] = u.z;
-            D[4 * k + 3] = u.w;
-          }
-        }
-      } else {
-  #pragma unroll
-        for (int k = 0; k < SH; ++k) D[k] = P::zero();
-      }
-
-      // -- reference strip into registers (after the row state: fewer live registers)
-      RV R[NWH];
-      if (p.use_tma) {
-        const int sl = s & 1;
-        // every lane waits (acquire of the TMA bytes); the give-up decision is warp-uniform
-        const bool ok = __all_sync(FULL_MASK, mbar_wait(&bars[sl], (phase >> sl) & 1u, spin_limit));
-        if (!ok) {
-          atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
-          return false;
-        }
-        phase ^= 1u << sl;
-        regs_from_smem<NWH, RV>(slot0 + sl * STRIP_BYTES, lane, R);
-        __syncwarp();
-        if (s + 1 < nstrips) {
-          const int ns = (s + 1) & 1;
-          fence_proxy_async_smem();
-          tma_issue_if(slot0 + ns * STRIP_BYTES, &tmap, &bars[ns], 0,
-                       (int)((ref_plane + (s + 1 < nh ? x + WH : a)) * RB / 128),
-                       STRIP_BYTES, is0);
-        }
-      } else if constexpr (PREC == 1) {
-        if (p.ref_layout == 0)
-          regs_from_pairs<SH>(reinterpret_cast<const float2 *>(p.ref_plain), x, lane, strand, R);
-        else
-          regs_from_global<NWH, RV>(reinterpret_cast<const float *>(p.ref_plain) + ref_plane + x, lane, R);
-      } else if constexpr (PREC == 2) {
-        regs_from_global<NWH, RV>(reinterpret_cast<const __half *>(p.ref_plain) + ref_plane + x, lane, R);
-      } else {
-        regs_from_global<NWH, RV>(reinterpret_cast<const __half2 *>(p.ref_plain) + x, lane, R);
-      }
-
-      // uniform stores (every lane writes the same value): no lane-dependent branch
-      seam_out[0] = P::shfl(D[SH - 1], 31);
-      if constexpr (PREC == 0) off_out[0] = O;
-
-      // offset of this strip's frame relative to the left strip's frame (FP16)
-      V delta = P::zero();
-      float2 off_next = make_float2(0.f, 0.f);
-      if constexpr (PREC == 0) {
-        if (!first) {
-          const float2 oi = off_in[0];
-          delta = __float22half2_rn(make_float2(oi.x - O.x, oi.y - O.y));
-          if (n >= K) off_next = off_in[1];
-        }
-      }
-
-      // -- row sweep, 32 rows per window: lane l holds query sample i0+l and
-      // the incoming seam value of row i0+l, already re-based into this strip's
-      // frame (delta changes only at a rescale, which ends a window)
-      const V vinf = P::inf();
-      typename P::QW qwin = P::qw(lane < n ? q[lane] : 0.f);
-      V swin = (!first && lane < rows) ? seam_in[lane] : vinf;
-      if constexpr (PREC == 0) swin = __hadd2(swin, delta);
-      V *so = seam_out + 1;  // seam value of row i goes to seam_out[i + 1]
-      for (int i0 = 0; i0 < rows; i0 += kWarp) {
-        const int r = i0 + kWarp + lane;
-        const float qn = r < n ? q[r] : 0.f;
-        const V sn = (!first && r < rows) ? seam_in[r] : vinf;
-        // the seam column leaving this strip is gathered in a register window
-        // (lane l keeps row i0+l) and stored once per 32 rows, coalesced: no
-        // lane-conditional store inside the row loop
-        V sout = vinf;
-        if (rows - i0 >= kWarp) {
-  #pragma unroll kRowUnroll
-          for (int il = 0; il < kWarp; ++il) {
-            row<SH, PREC>(D, R, P::qbcast(qwin, il), P::shfl(swin, il), m0);
-            if constexpr (SMEM_SEAM)
-              st_shared_if(sob + 4u * (uint32_t)il, cell_bits<PREC>(D[SH - 1]), is31);
-            else
-              sout = P::sel(lane == il, P::shfl(D[SH - 1], 31), sout);
-          }
-          if constexpr (PREC == 0) {
-            // rescale: subtract this strip's row minimum (one epoch = 32 rows)
-            V mn = D[0];
-  #pragma unroll
-            for (int k = 1; k < SH; ++k) mn = __hmin2(mn, D[k]);
-  #pragma unroll
-            for (int m = 16; m >= 1; m >>= 1) mn = __hmin2(mn, P::shfl_xor(mn, m));
-  #pragma unroll
-            for (int k = 0; k < SH; ++k) D[k] = __hsub2(D[k], mn);
-            const float2 mf = __half22float2(mn);
-            O.x += mf.x;
-            O.y += mf.y;
-            const int e = (i0 + kWarp) / K;
-            off_out[e] = O;  // warp-uniform value, stored by every lane
-            sout = P::sel(lane == kWarp - 1, P::shfl(D[SH - 1], 31), sout);  // the seam leaves in the new frame
-            if (!first) {
-              delta = __float22half2_rn(make_float2(off_next.x - O.x, off_next.y - O.y));
-              if ((e + 1) * K <= n) off_next = off_in[e + 1];
-            }
-          }
-          if constexpr (SMEM_SEAM) {
-            __syncwarp();
-            sout = P::from_bits(ld_shared_u32(sob + 4u * (uint32_t)lane));
-            __syncwarp();
-          }
-          so[lane] = sout;
-        } else {
-          const int cnt = rows - i0;
-          for (int il = 0; il < cnt; ++il) {
-            row<SH, PREC>(D, R, P::qbcast(qwin, il), P::shfl(swin, il), m0);
-            if constexpr (SMEM_SEAM)
-              st_shared_if(sob + 4u * (uint32_t)il, cell_bits<PREC>(D[SH - 1]), is31);
-            else
-              sout = P::sel(lane == il, P::shfl(D[SH - 1], 31), sout);
-          }
-          if constexpr (SMEM_SEAM) {
-            __syncwarp();
-            sout = lane < cnt ? P::from_bits(ld_shared_u32(sob + 4u * (uint32_t)lane)) : vinf;
-            __syncwarp();
-          }
-          so[lane] = sout;  // lanes >= cnt write +inf into the buffer's 32-entry slack past the rows
-        }
-        so += kWarp;
-        qwin = P::qw(qn);
-        swin = sn;
-        if constexpr (PREC == 0) swin = __hadd2(swin, delta);
-      }
-      if (rows < n) {
-        // rows this halo strip skipped can no longer reach column a: keep them
-        // inert (whole 32-entry groups; the buffers have 32 entries of slack)
-        for (int rr = rows + 1; rr <= n; rr += kWarp) seam_out[rr + lane] = vinf;
-        if constexpr (PREC == 0) {
-          for (int e = rows / K + 1; e <= n / K; e += kWarp) off_out[e + lane] = O;
-        }
-      }
-      __syncwarp();
-
-      return true;
-    };
-    if constexpr (SH != S) {
-      for (int s = 0; s < nh; ++s)
-        if (!sweep_halo_strip(s)) return;
+      const int64_t lim = (int64_t)n - 1 - (g.a - st.x - WH);
+      st.rows = (int)(lim < 0 ? 0 : (lim > n ? n : lim));
     }
+    st.strand = strand;
+    st.first = s == 0;
+    st.resume = (t.flags & kTaskResume) != 0;
+    st.q = p.query + t.q_off;
+    // planar row state: strand s of this read at state + state_off + s*m_pad
+    st.st_plane0 = p.state ? p.state + t.state_off : nullptr;
+    st.seq = seq;
+    const uint32_t buf = seq % (uint32_t)nbuf;
+    const uint32_t buf_in = buf ? buf - 1 : (uint32_t)nbuf - 1;
+    st.out_b = seam_base + buf * seam_half;
+    st.in_b = seam_base + buf_in * seam_half;
+    st.prog_out = prog + 8 * buf;
+    st.prog_in = prog + 8 * buf_in;
 
-    for (int s = s_main; s < nstrips; ++s) {
-      const int64_t x = xm0 + (int64_t)(s - s_main) * W;
-      const bool relevant = x >= a;
-      const bool first = (s == 0);
-      int rows = n;
-      if (!relevant) {
-        const int64_t lim = (int64_t)n - 1 - (a - x - W);
-        rows = (int)(lim < 0 ? 0 : (lim > n ? n : lim));
-      }
-
-      // -- seam buffers (ping-pong by strip parity)
-      char *in_b = seam_base + ((s + 1) & 1) * seam_half;
-      char *out_b = seam_base + (s & 1) * seam_half;
-      const V *seam_in = reinterpret_cast<const V *>(in_b);
-      const float2 *off_in = reinterpret_cast<const float2 *>(in_b + off_pos);
-      V *seam_out = reinterpret_cast<V *>(out_b);
-      float2 *off_out = reinterpret_cast<float2 *>(out_b + off_pos);
-
-      // -- initial row ("row -1"): zeros (free start) or the saved row state
-      V D[S];
-      float2 O = make_float2(0.f, 0.f);  // FP16 frame offsets (fwd, rev)
-      if (resume) {
-        const int64_t c0 = x + (int64_t)lane * S;
-        if constexpr (PREC == 0) {
-          if constexpr (ST16) {
-            // FP16 row state: half2 cells relative to the offset of their
-            // 512-column group (the saving strip's frame); re-based onto this
-            // strip's minimum
-            const uint4 *hc = reinterpret_cast<const uint4 *>(reinterpret_cast<const __half2 *>(st_plane0) + c0);
-            const float2 *og = reinterpret_cast<const float2 *>(st_plane0 + p.m_pad);
-#pragma unroll
-            for (int k = 0; k < S / 4; ++k) {
-              const uint4 u = hc[k];
-              D[4 * k] = bits_as<__half2>(u.x);
-              D[4 * k + 1] = bits_as<__half2>(u.y);
-              D[4 * k + 2] = bits_as<__half2>(u.z);
-              D[4 * k + 3] = bits_as<__half2>(u.w);
-            }
-            float mx = __int_as_float(0x7f800000), my = mx;
-#pragma unroll
-            for (int k = 0; k < S; ++k) {
-              const float2 o = og[(c0 + k) >> 9];
-              const float2 v = __half22float2(D[k]);
-              mx = fminf(mx, v.x + o.x);
-              my = fminf(my, v.y + o.y);
-            }
-#pragma unroll
-            for (int m = 16; m >= 1; m >>= 1) {
-              mx = fminf(mx, __shfl_xor_sync(FULL_MASK, mx, m));
-              my = fminf(my, __shfl_xor_sync(FULL_MASK, my, m));
-            }
-            O = make_float2(mx, my);
-#pragma unroll
-            for (int k = 0; k < S; ++k) {
-              const float2 o = og[(c0 + k) >> 9];
-              const float2 v = __half22float2(D[k]);
-              D[k] = __floats2half2_rn(v.x + o.x - mx, v.y + o.y - my);
-            }
-          } else {
-          // two passes over the saved planes: strip minimum first, then the cells
-          const float4 *f0 = reinterpret_cast<const float4 *>(st_plane0 + c0);
-          const float4 *f1 = reinterpret_cast<const float4 *>(st_plane0 + p.m_pad + c0);
-          float mx = __int_as_float(0x7f800000), my = mx;
-#pragma unroll
-          for (int k = 0; k < S / 4; ++k) {
-            const float4 u = f0[k], v = f1[k];
-            mx = fminf(mx, fminf(fminf(u.x, u.y), fminf(u.z, u.w)));
-            my = fminf(my, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
-          }
-#pragma unroll
-          for (int m = 16; m >= 1; m >>= 1) {
-            mx = fminf(mx, __shfl_xor_sync(FULL_MASK, mx, m));
-            my = fminf(my, __shfl_xor_sync(FULL_MASK, my, m));
-          }
-          O = make_float2(mx, my);
-#pragma unroll
-          for (int k = 0; k < S / 4; ++k) {
-            const float4 u = f0[k], v = f1[k];
-            D[4 * k] = __floats2half2_rn(u.x - mx, v.x - my);
-            D[4 * k + 1] = __floats2half2_rn(u.y - mx, v.y - my);
-            D[4 * k + 2] = __floats2half2_rn(u.z - mx, v.z - my);
-            D[4 * k + 3] = __floats2half2_rn(u.w - mx, v.w - my);
-          }
-          }
-        } else {
-          const float4 *f = reinterpret_cast<const float4 *>(st_plane0 + (int64_t)strand * p.m_pad + c0);
-#pragma unroll
-          for (int k = 0; k < S / 4; ++k) {
-            const float4 u = f[k];
-            D[4 * k] = u.x;
-            D[4 * k + 1] = u.y;
-            D[4 * k + 2] = u.z;
-            D[4 * k + 3] = u.w;
-          }
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < S; ++k) D[k] = P::zero();
-      }
-
-      // -- reference strip into registers (after the row state: fewer live registers)
-      RV R[NW];
-      if (p.use_tma) {
-        const int sl = s & 1;
-        // every lane waits (acquire of the TMA bytes); the give-up decision is warp-uniform
-        const bool ok = __all_sync(FULL_MASK, mbar_wait(&bars[sl], (phase >> sl) & 1u, spin_limit));
-        if (!ok) {
-          atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
-          return;
-        }
-        phase ^= 1u << sl;
-        regs_from_smem<NW, RV>(slot0 + sl * STRIP_BYTES, lane, R);
+    // the buffer's last writer and its reader (the strip after it) must be
+    // done; the reader may end first, where it begins another item
+    bool ok = true;
+    if (seq >= (uint32_t)nbuf) {
+      const uint32_t last = seq - (uint32_t)nbuf;
+      ok = team_wait(st.prog_out, ((uint64_t)(last + 1) << 32) | kWindowsDone, abort_a, p.max_rows) &&
+           team_wait(prog + 8 * ((buf + 1) % (uint32_t)nbuf), ((uint64_t)(last + 2) << 32) | kWindowsDone, abort_a,
+                     p.max_rows);
+    }
+    if (ok && p.use_tma) {
+      // the test hook p.stall_item withholds this copy (and its arrival) for
+      // one item's first strip: the wait for it then runs out with no copy in flight
+      const int64_t ref_plane = (PREC == 2 || (PREC == 1 && p.ref_layout == 1)) ? (int64_t)strand * p.m_pad : 0;
+      fence_proxy_async_smem();
+      tma_issue_if(slot, &tmap, bar, 0, (int)((ref_plane + st.x) * RB / 128), STRIP_BYTES,
+                   is0 & (s > 0 || item + 1 != p.stall_item ? 1u : 0u));
+    }
+    // a resumed halo strip counts itself in once it has read its row state
+    const auto on_loaded = [&]() {
+      if (halo && p.halo_read) {
+        __threadfence();
         __syncwarp();
-        if (s + 1 < nstrips) {
-          const int ns = (s + 1) & 1;
-          fence_proxy_async_smem();
-          tma_issue_if(slot0 + ns * STRIP_BYTES, &tmap, &bars[ns], 0, (int)((ref_plane + x + W) * RB / 128),
-                       STRIP_BYTES, is0);
-        }
-      } else if constexpr (PREC == 1) {
-        if (p.ref_layout == 0)
-          regs_from_pairs<S>(reinterpret_cast<const float2 *>(p.ref_plain), x, lane, strand, R);
-        else
-          regs_from_global<NW, RV>(reinterpret_cast<const float *>(p.ref_plain) + ref_plane + x, lane, R);
-      } else if constexpr (PREC == 2) {
-        regs_from_global<NW, RV>(reinterpret_cast<const __half *>(p.ref_plain) + ref_plane + x, lane, R);
-      } else {
-        regs_from_global<NW, RV>(reinterpret_cast<const __half2 *>(p.ref_plain) + x, lane, R);
+        red_add_if(&p.halo_read[item], 1, is0);
       }
+    };
 
-      // uniform stores (every lane writes the same value): no lane-dependent branch
-      seam_out[0] = P::shfl(D[S - 1], 31);
-      if constexpr (PREC == 0) off_out[0] = O;
-
-      // offset of this strip's frame relative to the left strip's frame (FP16)
-      V delta = P::zero();
-      float2 off_next = make_float2(0.f, 0.f);
-      if constexpr (PREC == 0) {
-        if (!first) {
-          const float2 oi = off_in[0];
-          delta = __float22half2_rn(make_float2(oi.x - O.x, oi.y - O.y));
-          if (n >= K) off_next = off_in[1];
-        }
+    bool swept = false;
+    if constexpr (SH != S) {
+      if (halo) {
+        V D[SH];
+        float2 O;
+        if (ok)
+          ok = sweep_strip<SH, PREC, ST16>(p, st, D, O, lane, m0, is31, wb, slot, bar, phase, spin_limit,
+                                                  abort_a, on_loaded);
+        swept = true;
       }
-
-      // -- row sweep, 32 rows per window: lane l holds query sample i0+l and
-      // the incoming seam value of row i0+l, already re-based into this strip's
-      // frame (delta changes only at a rescale, which ends a window)
-      const V vinf = P::inf();
-      typename P::QW qwin = P::qw(lane < n ? q[lane] : 0.f);
-      V swin = (!first && lane < rows) ? seam_in[lane] : vinf;
-      if constexpr (PREC == 0) swin = __hadd2(swin, delta);
-      V *so = seam_out + 1;  // seam value of row i goes to seam_out[i + 1]
-      for (int i0 = 0; i0 < rows; i0 += kWarp) {
-        const int r = i0 + kWarp + lane;
-        const float qn = r < n ? q[r] : 0.f;
-        const V sn = (!first && r < rows) ? seam_in[r] : vinf;
-        // the previous window of the incoming seam (entries i0-32 .. i0-1,
-        // one aligned 128-byte line of this warp's scratch) was consumed in
-        // the previous 32 rows: drop it from L2 instead of letting it be
-        // written back to DRAM.  Only in the batched FP16 instance, where long
-        // reads make the seam columns outgrow L2 (the other instances'
-        // register allocation suffers from it)
-        if constexpr (PREC == 0 && !NH && !ST16)
-          discard_l2_if(seam_in + i0 - kWarp, is0 & (!first && i0 > 0 ? 1u : 0u));
-        // the seam column leaving this strip is gathered in a register window
-        // (lane l keeps row i0+l) and stored once per 32 rows, coalesced: no
-        // lane-conditional store inside the row loop
-        V sout = vinf;
-        if (rows - i0 >= kWarp) {
-#pragma unroll kRowUnroll
-          for (int il = 0; il < kWarp; ++il) {
-            row<S, PREC>(D, R, P::qbcast(qwin, il), P::shfl(swin, il), m0);
-            if constexpr (SMEM_SEAM)
-              st_shared_if(sob + 4u * (uint32_t)il, cell_bits<PREC>(D[S - 1]), is31);
-            else
-              sout = P::sel(lane == il, P::shfl(D[S - 1], 31), sout);
-          }
+    }
+    if (!swept) {
+      V D[S];
+      float2 O;
+      if (ok)
+        ok = sweep_strip<S, PREC, ST16>(p, st, D, O, lane, m0, is31, wb, slot, bar,
+                                                                    phase, spin_limit, abort_a, on_loaded);
+      if (ok && !halo) {
+        const int64_t c0 = st.x + (int64_t)lane * S;
+        float bestx = __int_as_float(0x7f800000), besty = bestx;
+        int64_t colx = -1, coly = -1;
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+          const int64_t col = c0 + k;
           if constexpr (PREC == 0) {
-            // rescale: subtract this strip's row minimum (one epoch = 32 rows)
-            V mn = D[0];
-#pragma unroll
-            for (int k = 1; k < S; ++k) mn = __hmin2(mn, D[k]);
-#pragma unroll
-            for (int m = 16; m >= 1; m >>= 1) mn = __hmin2(mn, P::shfl_xor(mn, m));
-#pragma unroll
-            for (int k = 0; k < S; ++k) D[k] = __hsub2(D[k], mn);
-            const float2 mf = __half22float2(mn);
-            O.x += mf.x;
-            O.y += mf.y;
-            const int e = (i0 + kWarp) / K;
-            off_out[e] = O;  // warp-uniform value, stored by every lane
-            sout = P::sel(lane == kWarp - 1, P::shfl(D[S - 1], 31), sout);  // the seam leaves in the new frame
-            if (!first) {
-              delta = __float22half2_rn(make_float2(off_next.x - O.x, off_next.y - O.y));
-              if ((e + 1) * K <= n) off_next = off_in[e + 1];
-            }
-          }
-          if constexpr (SMEM_SEAM) {
-            __syncwarp();
-            sout = P::from_bits(ld_shared_u32(sob + 4u * (uint32_t)lane));
-            __syncwarp();
-          }
-          so[lane] = sout;
-        } else {
-          const int cnt = rows - i0;
-          for (int il = 0; il < cnt; ++il) {
-            row<S, PREC>(D, R, P::qbcast(qwin, il), P::shfl(swin, il), m0);
-            if constexpr (SMEM_SEAM)
-              st_shared_if(sob + 4u * (uint32_t)il, cell_bits<PREC>(D[S - 1]), is31);
-            else
-              sout = P::sel(lane == il, P::shfl(D[S - 1], 31), sout);
-          }
-          if constexpr (SMEM_SEAM) {
-            __syncwarp();
-            sout = lane < cnt ? P::from_bits(ld_shared_u32(sob + 4u * (uint32_t)lane)) : vinf;
-            __syncwarp();
-          }
-          so[lane] = sout;  // lanes >= cnt write +inf into the buffer's 32-entry slack past the rows
-        }
-        so += kWarp;
-        qwin = P::qw(qn);
-        swin = sn;
-        if constexpr (PREC == 0) swin = __hadd2(swin, delta);
-      }
-      if (rows < n) {
-        // rows this halo strip skipped can no longer reach column a: keep them
-        // inert (whole 32-entry groups; the buffers have 32 entries of slack)
-        for (int rr = rows + 1; rr <= n; rr += kWarp) seam_out[rr + lane] = vinf;
-        if constexpr (PREC == 0) {
-          for (int e = rows / K + 1; e <= n / K; e += kWarp) off_out[e + lane] = O;
-        }
-      }
-      __syncwarp();
-
-      if (relevant) {
-        const int64_t c0 = x + (int64_t)lane * S;
-        if constexpr (PREC == 0) {
-          if (ST16 && save) {
-            // half2 cells in this strip's frame, the frame offset once per 512-column group
-            uint4 *hc = reinterpret_cast<uint4 *>(reinterpret_cast<__half2 *>(p.state + t.state_off) + c0);
-#pragma unroll
-            for (int k = 0; k < S / 4; ++k)
-              hc[k] = make_uint4(cell_bits<0>(D[4 * k]), cell_bits<0>(D[4 * k + 1]), cell_bits<0>(D[4 * k + 2]),
-                                 cell_bits<0>(D[4 * k + 3]));
-            float2 *og = reinterpret_cast<float2 *>(p.state + t.state_off + p.m_pad);
-            og[c0 >> 9] = O;  // every lane of the strip stores the same value
-            og[(c0 + S - 1) >> 9] = O;
-          }
-#pragma unroll
-          for (int k = 0; k < S; ++k) {
             const float2 v = __half22float2(D[k]);
             const float vx = v.x + O.x, vy = v.y + O.y;
-            const int64_t col = c0 + k;
-            if (col < b) {
+            if (col < g.b) {
               if (vx < bestx) { bestx = vx; colx = col; }
               if (vy < besty) { besty = vy; coly = col; }
             }
+          } else {
+            if (col < g.b && D[k] < bestx) { bestx = D[k]; colx = col; }
           }
-          if (!ST16 && save) {
-            float4 *f0 = reinterpret_cast<float4 *>(p.state + t.state_off + c0);
-            float4 *f1 = reinterpret_cast<float4 *>(p.state + t.state_off + p.m_pad + c0);
-#pragma unroll
-            for (int k = 0; k < S / 4; ++k) {
-              const float2 v0 = __half22float2(D[4 * k]), v1 = __half22float2(D[4 * k + 1]);
-              const float2 v2 = __half22float2(D[4 * k + 2]), v3 = __half22float2(D[4 * k + 3]);
-              f0[k] = make_float4(v0.x + O.x, v1.x + O.x, v2.x + O.x, v3.x + O.x);
-              f1[k] = make_float4(v0.y + O.y, v1.y + O.y, v2.y + O.y, v3.y + O.y);
-            }
-          }
+        }
+        if (save) {
+          // wait for the halo strips of the chunks to the right that start from
+          // this strip's saved row (handed out before this chunk)
+          if (p.halo_read && st.resume) ok = wait_halo_readers<W, WH>(p, g, st.x, item, chunk, n, abort_a);
+          if (ok)
+            save_row_state<S, PREC, ST16>(D, O, p.state + t.state_off, p.m_pad, strand, c0);
+        }
+        warp_argmin(bestx, colx);
+        const int64_t base = 2 * (int64_t)t.out_slot;
+        if constexpr (PREC == 0) {
+          warp_argmin(besty, coly);
+          red_min_if(&p.keys[base + 0], make_key(bestx, colx), is0 & (colx >= 0 ? 1u : 0u));
+          red_min_if(&p.keys[base + 1], make_key(besty, coly), is0 & (coly >= 0 ? 1u : 0u));
         } else {
-#pragma unroll
-          for (int k = 0; k < S; ++k) {
-            const int64_t col = c0 + k;
-            if (col < b && D[k] < bestx) { bestx = D[k]; colx = col; }
-          }
-          if (save) {
-            float4 *f = reinterpret_cast<float4 *>(p.state + t.state_off + (int64_t)strand * p.m_pad + c0);
-#pragma unroll
-            for (int k = 0; k < S / 4; ++k) f[k] = make_float4(D[4 * k], D[4 * k + 1], D[4 * k + 2], D[4 * k + 3]);
-          }
+          red_min_if(&p.keys[base + strand], make_key(bestx, colx), is0 & (colx >= 0 ? 1u : 0u));
         }
       }
     }
-
-    warp_argmin(bestx, colx);
-    if constexpr (PREC == 0) warp_argmin(besty, coly);
-    {
-      const int64_t base = 2 * (int64_t)t.out_slot;
-      if constexpr (PREC == 0) {
-        red_min_if(&p.keys[base + 0], make_key(bestx, colx), is0 & (colx >= 0 ? 1u : 0u));
-        red_min_if(&p.keys[base + 1], make_key(besty, coly), is0 & (coly >= 0 ? 1u : 0u));
-      } else {
-        red_min_if(&p.keys[base + strand], make_key(bestx, colx), is0 & (colx >= 0 ? 1u : 0u));
-      }
+    if (!ok) {
+      atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
+      st_shared_volatile(abort_a, 1);
+      return;
     }
+    team_publish(st.prog_out, seq, kWindowsDone);
   }
 }
 
@@ -1039,7 +1110,8 @@ int sdtw_ref_bytes(int precision) { return precision == 2 ? 2 : 4; }
 
 size_t sdtw_smem_bytes(int precision, int cells_per_thread, int warps_per_cta) {
   const size_t strip = (size_t)kWarp * cells_per_thread * sdtw_ref_bytes(precision);
-  return 1024 /* alignment slack */ + 2 * warps_per_cta * strip + 16 * warps_per_cta + 128 * warps_per_cta;
+  // per warp: a strip tile, its mbarrier (16 bytes), three windows, two progress words; per CTA: the team's state
+  return 1024 /* alignment slack */ + warps_per_cta * (strip + 16 + 384 + 16) + kTeamStateBytes;
 }
 
 bool sdtw_instance_exists(int precision, int S, bool ref_del) {

@@ -134,7 +134,7 @@ extern "C" int dtwx_distances_static(const void *d_ref_pairs, int64_t ref_len, c
   if ((e = cudaMemcpyAsync(d_nsamp, h_nsamp, sizeof(int32_t) * n_reads, cudaMemcpyHostToDevice, st)) !=
       cudaSuccess)
     return st_fail(DTWX_E_CUDA, cudaGetErrorString(e));
-  if ((e = launch_reset(keys, 2 * n_reads, flags, flags + 4, st)) != cudaSuccess)
+  if ((e = launch_reset(keys, 2 * n_reads, flags, flags + 4, nullptr, 0, st)) != cudaSuccess)
     return st_fail(DTWX_E_CUDA, cudaGetErrorString(e));
   if (n_tasks) {
     SdtwParams p{};

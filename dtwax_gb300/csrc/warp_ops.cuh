@@ -19,6 +19,25 @@ __device__ __forceinline__ int ticket_if(int32_t *counter, uint32_t pred) {
   return v;
 }
 
+// Try-lock of a shared-memory word by the lanes whose pred is set: 0 = taken.
+__device__ __forceinline__ uint32_t lock_if(uint32_t addr, uint32_t pred) {
+  uint32_t v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u32 %0, 0;\n\t"
+      "@p atom.shared.cas.b32 %0, [%1], 0, 1;\n\t}"
+      : "=r"(v)
+      : "r"(addr), "r"(pred)
+      : "memory");
+  return v;
+}
+
+// 32-bit global add by the lanes whose pred is set.
+__device__ __forceinline__ void red_add_if(int32_t *addr, int32_t v, uint32_t pred) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p red.release.gpu.global.add.s32 [%0], %1;\n\t}" ::"l"(addr),
+               "r"(v), "r"(pred)
+               : "memory");
+}
+
 // 64-bit global min by the lanes whose pred is set, as predicated PTX.
 __device__ __forceinline__ void red_min_if(unsigned long long *addr, unsigned long long v, uint32_t pred) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p red.global.min.u64 [%0], %1;\n\t}" ::"l"(addr),
