@@ -42,6 +42,7 @@ struct Shape {
   int64_t items = 0;  // work items (while tuning: the candidate's chunk factor per mille)
   bool nh = false;  // narrow halo strips (FP16 pairs, narrow chunks)
   bool deal = false;  // items go to the CTAs in turn instead of first come, first served
+  uint64_t deal_warps = 0;  // deal: the warp of each strip of a CTA's first round, 4 bits each
 };
 
 // Buffers of one batch that may be in flight on its own stream.
@@ -304,14 +305,57 @@ double sweep_estimate(const RowCost &c, int64_t items, double work, double strip
 
 // Warps of a CTA (the team that sweeps an item's strips) when nothing fixes
 // them: all that fit on an SM, which leaves the fewest idle at the end of a
-// batch (5 Mb, 96 uneven reads: 246 ms, 291 with 2-warp teams).  4-warp teams
-// for reads too short to keep a long pipeline full (176 reads of 369 samples:
-// 459 against 490 us), and for FP16 batches of many items, where nothing is
-// left of the first reason and the shorter pipeline waits less (1.3 %).
-int default_team(int precision, int full, double mean_rows, int64_t items, int sms) {
-  if (mean_rows < 640) return 4;
-  if (precision == 0 && items >= (int64_t)8 * sms * (full / 4)) return 4;
-  return full;
+// batch (5 Mb, 96 uneven reads: 246 ms, 291 with 2-warp teams).  Fewer where a
+// read is too short to keep a long pipeline full: a strip of w windows starts
+// w / k windows behind its left neighbour, and below about 8 the two get in
+// each other's way (1,500 reads of 250 samples against 48 kb, G = 4: k = 1
+// 2.64, 2 2.88, 4 3.27 ms; 300 of 200 against 200 kb, G = 22: 1.58, 1.52,
+// 1.66).  With one or two strips to an item and short reads one warp does best
+// (300 of 700 against 9 kb: 0.354 ms, 12 warps 0.459).  FP16 batches of many
+// items take 4, where nothing is left of the first reason (1.3 %).
+// G: strips of a chunk.
+int default_team(int precision, int full, double mean_rows, int64_t items, int G, int sms) {
+  if (precision != 0) return mean_rows < 384 ? 1 : (mean_rows < 640 ? 4 : full);
+  if (mean_rows < 384) return G <= 2 || items >= (int64_t)20 * sms ? 1 : 2;
+  if (mean_rows < 800) return G <= 2 ? 1 : 4;
+  if (G == 1 && items > (int64_t)sms) {
+    // one own strip to an item, the rest narrow halo: a team's strips differ in
+    // weight and do not spread evenly over the schedulers (1.4 times the work's
+    // time); single warps do, at the price of a last round that is not full
+    // (1,638 items of 2,048 rows: 1.33 ms against 1.49; 702: 0.92 against 0.77)
+    const double w = std::ceil((double)items / (4.0 * sms));
+    const double alone = std::max(1.05 * 265.0, std::min(w, 3.0) * 217.0) * std::ceil(w / 3.0);
+    if (alone <= 1.4 * 217.0 * (double)items / (4.0 * sms)) return 1;
+  }
+  return items >= (int64_t)8 * sms * (full / 4) ? 4 : full;
+}
+
+// Which warp of a CTA takes the p-th strip of a dealt batch's first round
+// (4 bits per strip): heavy strips (the chunk's own, S cells per lane) and
+// narrow halo strips spread evenly over the SM's four schedulers (warp w runs
+// on scheduler w mod 4), largest first.
+uint64_t deal_warps(int warps, int nh, int g, int S, int SH, double rows, int WH) {
+  double weight[16], load[4] = {0, 0, 0, 0};
+  int order[16], used[4] = {0, 0, 0, 0};
+  const int per = nh + g;
+  for (int p = 0; p < warps; ++p) {
+    const int s = p % per;
+    // rows of halo strip s: those that still reach the chunk
+    const double r = s < nh ? std::max(1.0, std::min(rows, rows - (double)s * WH)) : rows;
+    weight[p] = r * (s < nh ? SH : S);
+    order[p] = p;
+  }
+  std::stable_sort(order, order + warps, [&](int a, int b) { return weight[a] > weight[b]; });
+  uint64_t map = 0;
+  for (int i = 0; i < warps; ++i) {
+    const int p = order[i];
+    int best = -1;
+    for (int q = 0; q < 4; ++q)
+      if (4 * used[q] + q < warps && (best < 0 || load[q] < load[best])) best = q;
+    load[best] += weight[p];
+    map |= (uint64_t)(4 * used[best]++ + best) << (4 * p);
+  }
+  return map;
 }
 
 // Launch shape of a sweep: user-fixed fields win, then an autotuned entry for
@@ -341,18 +385,18 @@ Shape pick_shape(dtwx_handle *h, int precision, int64_t n_tasks, double mean_row
   if (use_t && !f.G) g_scale = t->second.g_scale;
   if (o.S) g_scale = o.items > 0 ? o.items / 1000.0 : 1.0;  // candidate factor (per mille) while tuning
   int occ = std::max(1, sdtw_ctas_per_sm(precision, s.S, s.warps, rd));
-  if (!rd && precision != 0 && !o.S && !use_t && !f.G && auto_warps) {
+  if (!rd && precision != 0 && !o.S && !use_t && !f.G && auto_warps && mean_rows >= 384) {
     // FP32 path cost: any strip width and any chunks give the same bits, so the
-    // estimate picks both
+    // estimate picks both (reads too short for teams keep the model below)
     double best = 1e300;
     for (const RowCost &c : kRowCost[precision]) {
       if (f.S && c.S != f.S) continue;
       const int full = 4 * sdtw_ctas_per_sm(precision, c.S, 4, rd);
       if (full <= 0 || sdtw_ctas_per_sm(precision, c.S, full, rd) < 1) continue;
-      const int k = default_team(precision, full, mean_rows, 0, h->sms);
-      const int64_t teams = (int64_t)h->sms * full / k;
       const int W = kWarp * c.S;
       const int64_t strips = (h->m_cols + W - 1) / W;
+      const int k = default_team(precision, full, mean_rows, 0, 0, h->sms);
+      const int64_t teams = (int64_t)h->sms * full / k;
       int64_t chunks = 0;
       for (int64_t g = 1; g <= strips; g = chunks > 1 ? (strips + chunks - 2) / (chunks - 1) : g + 1) {
         chunks = (strips + g - 1) / g;
@@ -389,24 +433,36 @@ Shape pick_shape(dtwx_handle *h, int precision, int64_t n_tasks, double mean_row
   const int64_t chunks = (strips + s.G - 1) / s.G;
   s.nh = precision == 0 && !rd && chunks > 1 && s.G <= kNarrowHaloMaxStrips && s.S % kNarrowHaloCells == 0;
   s.items = n_tasks * chunks * strands;
-  if (auto_warps && (precision == 0 || s.warps == 4)) {
-    const int full = occ * s.warps;
-    const int k = default_team(precision, full, mean_rows, s.items, h->sms);
-    if (k != s.warps && sdtw_ctas_per_sm(precision, s.S, k, false) >= 1) {
-      s.warps = k;
-      occ = full / k;
-    }
-  }
   if (rd) {
     const int64_t want = (s.items + s.warps - 1) / s.warps;
     s.grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)h->sms * occ, want));
-  } else {
-    s.grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)h->sms * occ, s.items));
-    // when every strip of the batch can run at once, deal the items out evenly:
-    // the CTAs that start first would take more than their share
-    const int64_t halo_strips = chunks > 1 ? (int64_t)std::ceil(mean_rows / (s.nh ? kWarp * kNarrowHaloCells : W)) : 0;
-    s.deal = s.items * (s.G + halo_strips) <= (int64_t)s.grid * s.warps * 3 / 2;
+    return s;
   }
+  const int SH = s.nh ? kNarrowHaloCells : s.S;
+  const int nh = chunks > 1 ? (int)std::min<double>(1e6, std::ceil(mean_rows / (kWarp * SH))) : 0;
+  if (auto_warps) {
+    const int full = occ * s.warps;
+    // a batch whose strips can all run at once: one CTA per SM, its items dealt
+    // out in turn (first come, first served, the CTAs that start first take more
+    // than their share) and its strips placed by weight.  (10 reads of 2,048
+    // samples against 48 kb: 0.39 ms, 0.52 without.)  Batches of very short reads
+    // are over before the first round's bookkeeping pays
+    const int64_t strips_all = s.items * ((int64_t)s.G + nh);
+    if ((precision != 0 || s.nh) && full <= 16 && strips_all <= (int64_t)h->sms * full * 3 / 2 &&
+        (mean_rows >= 384 || s.items <= h->sms) && sdtw_ctas_per_sm(precision, s.S, full, false) >= 1) {
+      s.deal = true;
+      s.warps = full;
+      occ = 1;
+      s.deal_warps = deal_warps(full, nh, s.G, s.S, SH, mean_rows, kWarp * SH);
+    } else if (precision == 0 || mean_rows < 384) {
+      const int k = default_team(precision, full, mean_rows, s.items, s.G, h->sms);
+      if (k != s.warps && sdtw_ctas_per_sm(precision, s.S, k, false) >= 1) {
+        s.warps = k;
+        occ = full / k;
+      }
+    }
+  }
+  s.grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)h->sms * occ, s.items));
   return s;
 }
 
@@ -477,6 +533,7 @@ int enqueue_sweep(dtwx_handle *h, BatchCtx &c, int precision, cudaStream_t st, c
     p.state_fp16 = state_fp16(h) ? 1 : 0;
     p.narrow_halo = sh.nh ? 1 : 0;
     p.deal = sh.deal ? 1 : 0;
+    p.deal_warps = sh.deal_warps;
     p.stall_item = h->stall_item;
     p.spin_limit = h->stall_spin;
     h->stall_item = 0;
@@ -748,7 +805,9 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
       p.ref_layout = 1;
       p.narrow_halo = sh.nh ? 1 : 0;
       p.deal = sh.deal ? 1 : 0;
+      p.deal_warps = sh.deal_warps;
     p.deal = sh.deal ? 1 : 0;
+    p.deal_warps = sh.deal_warps;
         const int ii = inst_index(precision, sh.S);
       p.use_tma = h->tmap_ok[precision][ii] ? 1 : 0;
       CK(h, launch_sdtw(precision, sh.S, sh.warps, sh.grid, p, p.use_tma ? &h->tmap[precision][ii] : nullptr,

@@ -89,6 +89,7 @@ struct SdtwParams {
                                // frame offset per 512-column group (m_pad / 512)
   int32_t narrow_halo;         // FP16 pairs: launch the instance with kNarrowHaloCells-wide halo strips
   int32_t deal;                // 1: CTA b takes items b, b + grid, ...; 0: the next ticket of `counter`
+  uint64_t deal_warps;         // deal: the warp that takes the p-th strip of the CTA's first round, 4 bits each
   uint32_t spin_limit;         // polls before a bounded wait gives up; 0 = kSpinLimit
   int32_t stall_item;          // test hook: 1 + the queue ticket whose first reference-strip copy
                                // is not issued, so that its warp's bounded wait runs out; 0 = none

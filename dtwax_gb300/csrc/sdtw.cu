@@ -852,6 +852,9 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
   constexpr int STRIP_BYTES = W * RB;
   constexpr int SH = NH ? kNarrowHaloCells : S;  // cells per lane in halo strips
   constexpr int WH = kWarp * SH;
+  // dealt batches (p.deal): not in the FP16 instance of wide chunks, which has
+  // many items and whose rows lose 6 % to the registers of the first round
+  constexpr bool DEAL = PREC != 0 || NH;
   static_assert(S % SH == 0 && SH % 8 == 0, "halo strips must tile the chunk start");
   static_assert(!NH || PREC == 0, "narrow halo strips are built for FP16 pairs");
   static_assert(STRIP_BYTES % 1024 == 0, "strip tile must keep 1024-byte alignment");
@@ -898,55 +901,100 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
   const int64_t n_items = (int64_t)p.n_tasks * per_task;
   const uint32_t spin_limit = p.spin_limit ? p.spin_limit : kSpinLimit;
 
+  // Strips of an item (none of one with nothing to do or that is refused).
+  const auto item_strips = [&](int item) -> int {
+    const int tr = item / per_task;
+    const int n = p.tasks[p.order ? p.order[tr] : tr].n;
+    if (n <= 0 || n > p.max_rows) {
+      if (n > p.max_rows) atomicOr(p.err, kErrBadTask);  // every lane: same bit
+      return 0;
+    }
+    const int rem = item - tr * per_task;
+    return item_geometry<W, WH>(p, p.n_chunks - 1 - (!PAIRS ? rem % p.n_chunks : rem), n).nstrips;
+  };
+
+  // A dealt batch's first round: warp w takes the strip that p.deal_warps
+  // gives it, walking the CTA's items to find it; the warp with the last one
+  // leaves the cursor behind it.
+  int first_item = -1, first_s = 0;
+  uint32_t first_seq = 0;
+  if (DEAL && p.deal) {
+    int pos = 0;
+    while (pos < 15 && (int)((p.deal_warps >> (4 * pos)) & 15u) != warp) ++pos;
+    int at = 0, total = 0, dealt = 0;
+    int64_t item = blockIdx.x;
+    for (; item < n_items; item += gridDim.x) {
+      ++dealt;
+      total = item_strips((int)item);
+      if (pos < at + total) break;
+      at += total;
+    }
+    if (item < n_items) {
+      first_item = (int)item;
+      first_s = pos - at;
+      first_seq = (uint32_t)pos;
+    } else {
+      first_item = (int)n_items;  // fewer strips than warps
+    }
+    if (pos == nwarps - 1) {
+      st_shared_volatile(item_a, (uint32_t)first_item);
+      st_shared_volatile(next_a, (uint32_t)(first_s + 1));
+      st_shared_volatile(total_a, (uint32_t)total);
+      st_shared_volatile(seq_a, (uint32_t)nwarps);
+      st_shared_volatile(dealt_a, (uint32_t)dealt);
+    }
+    __syncthreads();
+  }
+
   for (;;) {
     // -- the next strip of the CTA's sequence, under the team's lock.  Every
     // lane runs the same instructions (only the atomics are lane 0's).
-    bool held = false;
-    for (uint32_t it = 0; it < (1u << 22) && !held; ++it) {
-      held = __shfl_sync(FULL_MASK, lock_if(lock_a, is0), 0) == 0;
-      if (!held) __nanosleep(20);
+    int item = -1, s = 0;
+    uint32_t seq = 0;
+    if constexpr (DEAL) {
+      item = first_item, s = first_s, seq = first_seq;
+      first_item = -1;
     }
-    __threadfence_block();
-    if (!held || __any_sync(FULL_MASK, ld_shared_volatile(abort_a) != 0)) {
-      atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
-      st_shared_volatile(abort_a, 1);
-      if (held) st_shared_volatile(lock_a, 0);
-      return;
-    }
-    int item = (int)ld_shared_volatile(item_a);
-    int s = (int)ld_shared_volatile(next_a);
-    int total = (int)ld_shared_volatile(total_a);
-    const uint32_t seq = ld_shared_volatile(seq_a);
-    while (s >= total && item < n_items) {
-      if (p.deal) {
-        const uint32_t dealt = ld_shared_volatile(dealt_a);
-        item = (int)(blockIdx.x + dealt * gridDim.x);
-        __syncwarp();
-        st_shared_volatile(dealt_a, dealt + 1);
-        __syncwarp();
-      } else {
-        item = __shfl_sync(FULL_MASK, ticket_if(p.counter, is0), 0);
+    if (item < 0) {
+      bool held = false;
+      for (uint32_t it = 0; it < (1u << 22) && !held; ++it) {
+        held = __shfl_sync(FULL_MASK, lock_if(lock_a, is0), 0) == 0;
+        if (!held) __nanosleep(20);
       }
-      if (item >= n_items) break;
-      const int tr = item / per_task;
-      const int n = p.tasks[p.order ? p.order[tr] : tr].n;
-      if (n <= 0 || n > p.max_rows) {
-        if (n > p.max_rows) atomicOr(p.err, kErrBadTask);  // every lane: same bit
-        continue;
+      __threadfence_block();
+      if (!held || __any_sync(FULL_MASK, ld_shared_volatile(abort_a) != 0)) {
+        atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
+        st_shared_volatile(abort_a, 1);
+        if (held) st_shared_volatile(lock_a, 0);
+        return;
       }
-      const int rem = item - tr * per_task;
-      const int chunk = p.n_chunks - 1 - (!PAIRS ? rem % p.n_chunks : rem);
-      s = 0;
-      total = item_geometry<W, WH>(p, chunk, n).nstrips;
+      item = (int)ld_shared_volatile(item_a);
+      s = (int)ld_shared_volatile(next_a);
+      int total = (int)ld_shared_volatile(total_a);
+      seq = ld_shared_volatile(seq_a);
+      while (s >= total && item < n_items) {
+        if (DEAL && p.deal) {
+          const uint32_t dealt = ld_shared_volatile(dealt_a);
+          item = (int)(blockIdx.x + dealt * gridDim.x);
+          __syncwarp();
+          st_shared_volatile(dealt_a, dealt + 1);
+          __syncwarp();
+        } else {
+          item = __shfl_sync(FULL_MASK, ticket_if(p.counter, is0), 0);
+        }
+        if (item >= n_items) break;
+        s = 0;
+        total = item_strips(item);
+      }
+      __syncwarp();
+      st_shared_volatile(item_a, (uint32_t)(item < n_items ? item : (int)n_items));
+      st_shared_volatile(next_a, (uint32_t)(s + 1));
+      st_shared_volatile(total_a, (uint32_t)total);
+      st_shared_volatile(seq_a, seq + 1);
+      __threadfence_block();
+      __syncwarp();
+      st_shared_volatile(lock_a, 0);
     }
-    __syncwarp();
-    st_shared_volatile(item_a, (uint32_t)(item < n_items ? item : (int)n_items));
-    st_shared_volatile(next_a, (uint32_t)(s + 1));
-    st_shared_volatile(total_a, (uint32_t)total);
-    st_shared_volatile(seq_a, seq + 1);
-    __threadfence_block();
-    __syncwarp();
-    st_shared_volatile(lock_a, 0);
     if (item >= n_items) break;
 
     const int tr = item / per_task;
