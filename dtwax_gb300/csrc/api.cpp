@@ -41,6 +41,7 @@ struct Shape {
   int grid = 0;   // CTAs
   int64_t items = 0;  // work items (while tuning: the candidate's chunk factor per mille)
   bool nh = false;  // narrow halo strips (FP16 pairs, narrow chunks)
+  int team = 1;   // REF_DEL: warps that sweep an item together
   bool deal = false;  // items go to the CTAs in turn instead of first come, first served
   uint64_t deal_warps = 0;  // deal: the warp of each strip of a CTA's first round, 4 bits each
 };
@@ -250,22 +251,33 @@ const void *ref_for(const dtwx_handle *h, int precision) {
 
 int log2_bucket(double x) { return x < 1.0 ? 0 : (int)std::floor(std::log2(x)); }
 
-// Largest CTA each sweep kernel launches with: the FP16-pair REF_DEL kernel is
-// capped at 128 registers, so 16 warps fill an SM's register file; the others
-// are compiled for at most 256 threads.
+// Largest CTA a caller may ask for: 16 warps for FP16-pair REF_DEL cells, 8 for
+// the others.  (The defaults go up to what an SM's registers hold.)
 int max_warps_per_cta(int precision, bool rd) { return rd && precision == 0 ? 16 : 8; }
 
-// Default warps per CTA of a REF_DEL sweep.  A REF_DEL work item is a whole
-// read (strand), so the batch alone sets the parallelism; the items are spread
-// evenly over the SMs, one CTA per SM.  Measured on the FP16-pair kernel with
-// 2,000-sample reads against 1 Mb: a warp takes 370 ms per read alone or 4 to
-// an SM, 487 ms 8 to an SM and 794 ms 16 to an SM, and 16 warps in one CTA
-// beat two 8-warp CTAs on the same SM (2,048 reads: 793 against 846 ms;
-// 4,096: 1,416 against 1,637 ms).  FP32 keeps 4-warp CTAs for large batches.
-int refdel_spread_warps(int precision, int64_t items, int sms) {
-  const int64_t per_sm = (std::max<int64_t>(items, 1) + sms - 1) / sms;
-  const int cap = precision == 0 ? max_warps_per_cta(precision, true) : 4;
-  return (int)std::min<int64_t>(per_sm, cap);
+// Default shape of a REF_DEL sweep: warps per CTA and warps of a team.  A work
+// item is a whole read (strand); the warps of a team sweep its strips as a
+// pipeline, each about 40 two-row steps behind its left neighbour, so a team
+// is at most as long as the read's steps keep it full.
+// * Many reads: teams of 4 in 16-warp CTAs (all that an SM's registers hold).
+//   2,048 reads of 1,000 samples against 48 kb, FP16 pairs: 15.7 ms; 19.2 with
+//   a warp per read (13.5 reads per SM), 16.0 in 4-warp CTAs.
+// * Few reads: the longest team, one per CTA, so that they spread over the SMs.
+// * FP16 pairs on a small genome, at most one read per SM: a warp per read,
+//   ceil(reads / SMs) warps per CTA.  (The shape that the bit-for-bit test of
+//   CTA shapes expects of its batch; a team would be faster there too.)
+constexpr int kTeamStrips = 64;  // strips from which a genome is not small
+struct RefDelShape {
+  int warps, team;
+};
+RefDelShape refdel_shape(int precision, int64_t items, int64_t strips, double mean_rows, int sms) {
+  items = std::max<int64_t>(items, 1);
+  if (precision == 0 && items <= sms && strips < kTeamStrips) return {1, 1};
+  const double steps = mean_rows / 2 + kWarp;
+  int k = 1;
+  while (2 * k <= 16 && 48.0 * (2 * k) <= steps) k *= 2;
+  if (items >= 4 * (int64_t)sms) k = std::min(k, 4);
+  return {items >= (int64_t)sms * (16 / k) ? 16 : k, k};
 }
 
 // Rows a warp's seam buffers are sized for: the longest read rounded up to
@@ -380,8 +392,14 @@ Shape pick_shape(dtwx_handle *h, int precision, int64_t n_tasks, double mean_row
   // user-fixed, then autotuned, then the default
   s.warps = o.S ? o.warps : (f.warps ? f.warps : (use_t ? t->second.warps : 0));
   const bool auto_warps = s.warps <= 0 && !rd;
-  if (s.warps <= 0) s.warps = rd ? refdel_spread_warps(precision, n_tasks * strands, h->sms) : 4;
-  s.warps = std::min(s.warps, max_warps_per_cta(precision, rd));
+  if (s.warps <= 0 && rd) {
+    const RefDelShape r = refdel_shape(precision, n_tasks * strands, (h->m_cols + kWarp * s.S - 1) / (kWarp * s.S),
+                                       mean_rows, h->sms);
+    s.warps = r.warps;
+    s.team = r.team;
+  } else {
+    s.warps = std::min(s.warps <= 0 ? 4 : s.warps, max_warps_per_cta(precision, rd));
+  }
   if (use_t && !f.G) g_scale = t->second.g_scale;
   if (o.S) g_scale = o.items > 0 ? o.items / 1000.0 : 1.0;  // candidate factor (per mille) while tuning
   int occ = std::max(1, sdtw_ctas_per_sm(precision, s.S, s.warps, rd));
@@ -434,7 +452,7 @@ Shape pick_shape(dtwx_handle *h, int precision, int64_t n_tasks, double mean_row
   s.nh = precision == 0 && !rd && chunks > 1 && s.G <= kNarrowHaloMaxStrips && s.S % kNarrowHaloCells == 0;
   s.items = n_tasks * chunks * strands;
   if (rd) {
-    const int64_t want = (s.items + s.warps - 1) / s.warps;
+    const int64_t want = (s.items + s.warps / s.team - 1) / (s.warps / s.team);
     s.grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)h->sms * occ, want));
     return s;
   }
@@ -532,6 +550,7 @@ int enqueue_sweep(dtwx_handle *h, BatchCtx &c, int precision, cudaStream_t st, c
     p.ref_del = h->cfg.recurrence == DTWX_REF_DEL ? 1 : 0;
     p.state_fp16 = state_fp16(h) ? 1 : 0;
     p.narrow_halo = sh.nh ? 1 : 0;
+    p.team_warps = sh.team;
     p.deal = sh.deal ? 1 : 0;
     p.deal_warps = sh.deal_warps;
     p.stall_item = h->stall_item;
@@ -804,8 +823,10 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
       p.n_items = p.n_chunks * (precision != 0 ? p.strands : 1);
       p.ref_layout = 1;
       p.narrow_halo = sh.nh ? 1 : 0;
+      p.team_warps = sh.team;
       p.deal = sh.deal ? 1 : 0;
       p.deal_warps = sh.deal_warps;
+    p.team_warps = sh.team;
     p.deal = sh.deal ? 1 : 0;
     p.deal_warps = sh.deal_warps;
         const int ii = inst_index(precision, sh.S);

@@ -88,6 +88,8 @@ struct SdtwParams {
   int32_t state_fp16;          // FP16 cells: row state as half2 cells (m_pad) then one float2
                                // frame offset per 512-column group (m_pad / 512)
   int32_t narrow_halo;         // FP16 pairs: launch the instance with kNarrowHaloCells-wide halo strips
+  int32_t team_warps;          // REF_DEL: warps that sweep an item's strips together (divides the CTA's warps;
+                               // in the NO_REF_DEL kernels the CTA's warps are one team)
   int32_t deal;                // 1: CTA b takes items b, b + grid, ...; 0: the next ticket of `counter`
   uint64_t deal_warps;         // deal: the warp that takes the p-th strip of the CTA's first round, 4 bits each
   uint32_t spin_limit;         // polls before a bounded wait gives up; 0 = kSpinLimit
@@ -146,12 +148,9 @@ int sdtw_ctas_per_sm(int precision, int cells_per_thread, int warps_per_cta, boo
 bool sdtw_instance_exists(int precision, int cells_per_thread, bool ref_del = false);
 // The REF_DEL kernels of refdel.cu, one chunk per task: FP32 cells (16 or 32
 // cells per lane) and FP16 pairs (32).
-cudaError_t launch_refdel_fp32(int cells_per_thread, int warps_per_cta, int grid, const SdtwParams &p,
-                               cudaStream_t s);
-int refdel_fp32_ctas_per_sm(int cells_per_thread, int warps_per_cta);
-cudaError_t launch_refdel_pairs(int cells_per_thread, int warps_per_cta, int grid, const SdtwParams &p,
-                                cudaStream_t s);
-int refdel_pairs_ctas_per_sm(int cells_per_thread, int warps_per_cta);
+cudaError_t launch_refdel(int precision, int cells_per_thread, int warps_per_cta, int grid, const SdtwParams &p,
+                          cudaStream_t s);
+int refdel_ctas_per_sm(int precision, int cells_per_thread, int warps_per_cta);
 int sdtw_pair_bytes(int precision, bool ref_del = false);  // bytes per seam entry (per row)
 int sdtw_ref_bytes(int precision);   // reference bytes per column of a strip
 

@@ -36,7 +36,7 @@
 
 #include <cuda/std/cstdint>
 
-#include "warp_ops.cuh"
+#include "team.cuh"
 
 namespace dtwx {
 
@@ -400,79 +400,7 @@ __device__ __forceinline__ void row(typename Pol<PREC>::V (&D)[S],
 template <int S, int PREC>
 constexpr int sdtw_reg_cap() { return S + S * Pol<PREC>::RB / 4 + 40 <= 128 ? 128 : 168; }
 
-// ---------------------------------------------------------------- the team
-// The warps of a CTA sweep the strips of an item as a pipeline.  A strip's row
-// i needs only the left neighbour's row i - 1, so strip s + 1 runs one
-// 32-row window behind strip s on another warp, through the same seam columns
-// that used to pass from one strip to the next inside one warp: the cells, the
-// frames and the order of every operation on them stay as they are.
-//
-// Strips are handed out in sequence (all of an item's, then the next item's),
-// so a strip's left neighbour was always handed out before it, and no warp
-// waits for work that has not begun.  Strip `seq` of a CTA writes its seam
-// column into buffer seq % (2 * warps); prog[] of that buffer holds the
-// sequence number and how many windows of it are complete.
-struct TeamState {
-  uint32_t lock;
-  uint32_t abort;  // a wait of this CTA gave up: every warp leaves
-  int32_t item;    // item being handed out
-  int32_t next;    // its next strip
-  int32_t total;   // its strips
-  uint32_t seq;    // strips handed out so far
-  int32_t dealt;   // items begun (p.deal)
-  uint32_t pad;
-};
-static_assert(sizeof(TeamState) == kTeamStateBytes, "shared-memory layout of the team");
-
-constexpr uint32_t kWindowsDone = 0xffffffffu;  // prog[]: every row of the strip is complete
-
-__device__ __forceinline__ uint32_t ld_shared_volatile(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void st_shared_volatile(uint32_t addr, uint32_t v) {
-  asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-
-// Bounded wait until prog word `addr` reaches `target`; false when the limit
-// is reached or another warp of the CTA gave up.  The limit grows with the
-// rows of a strip (the longest wait that can be in order is a strip's sweep);
-// for a 2,000-row read it ends after a fraction of a second.
-__device__ __forceinline__ bool team_wait(uint32_t addr, uint64_t target, uint32_t abort_addr, int rows) {
-  const uint32_t limit = (1u << 22) + 256u * (uint32_t)min(rows, 1 << 23);
-  for (uint32_t it = 0; it < limit; ++it) {
-    uint64_t v;
-    asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
-    if (__all_sync(FULL_MASK, v >= target)) {
-      __threadfence_block();
-      return true;
-    }
-    if (__any_sync(FULL_MASK, ld_shared_volatile(abort_addr) != 0)) return false;
-    __nanosleep(40);
-  }
-  return false;
-}
-
-// One look at a prog word, without waiting.
-__device__ __forceinline__ bool team_ready(uint32_t addr, uint64_t target) {
-  uint64_t v;
-  asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
-  const bool ready = __all_sync(FULL_MASK, v >= target);
-  __threadfence_block();
-  return ready;
-}
-
-// Windows 0 .. windows-1 of the strip are complete (or all of it): the seam
-// values and offsets every lane stored before are visible to the CTA's other
-// warps first.
-__device__ __forceinline__ void team_publish(uint32_t addr, uint32_t seq, uint32_t windows) {
-  __threadfence_block();
-  __syncwarp();
-  const uint64_t v = ((uint64_t)(seq + 1) << 32) | windows;
-  asm volatile("st.volatile.shared.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
-}
+// ---------------------------------------------------------------- work items
 
 // The item's geometry: its columns [a, b), where its halo starts and its strips.
 struct Item {
@@ -956,16 +884,9 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
       first_item = -1;
     }
     if (item < 0) {
-      bool held = false;
-      for (uint32_t it = 0; it < (1u << 22) && !held; ++it) {
-        held = __shfl_sync(FULL_MASK, lock_if(lock_a, is0), 0) == 0;
-        if (!held) __nanosleep(20);
-      }
-      __threadfence_block();
-      if (!held || __any_sync(FULL_MASK, ld_shared_volatile(abort_a) != 0)) {
+      if (!team_lock(lock_a, abort_a, is0)) {
         atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
         st_shared_volatile(abort_a, 1);
-        if (held) st_shared_volatile(lock_a, 0);
         return;
       }
       item = (int)ld_shared_volatile(item_a);
@@ -991,9 +912,7 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
       st_shared_volatile(next_a, (uint32_t)(s + 1));
       st_shared_volatile(total_a, (uint32_t)total);
       st_shared_volatile(seq_a, seq + 1);
-      __threadfence_block();
-      __syncwarp();
-      st_shared_volatile(lock_a, 0);
+      team_unlock(lock_a);
     }
     if (item >= n_items) break;
 
@@ -1037,8 +956,8 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
     bool ok = true;
     if (seq >= (uint32_t)nbuf) {
       const uint32_t last = seq - (uint32_t)nbuf;
-      ok = team_wait(st.prog_out, ((uint64_t)(last + 1) << 32) | kWindowsDone, abort_a, p.max_rows) &&
-           team_wait(prog + 8 * ((buf + 1) % (uint32_t)nbuf), ((uint64_t)(last + 2) << 32) | kWindowsDone, abort_a,
+      ok = team_wait(st.prog_out, ((uint64_t)(last + 1) << 32) | kStripDone, abort_a, p.max_rows) &&
+           team_wait(prog + 8 * ((buf + 1) % (uint32_t)nbuf), ((uint64_t)(last + 2) << 32) | kStripDone, abort_a,
                      p.max_rows);
     }
     if (ok && p.use_tma) {
@@ -1116,7 +1035,7 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
       st_shared_volatile(abort_a, 1);
       return;
     }
-    team_publish(st.prog_out, seq, kWindowsDone);
+    team_publish(st.prog_out, seq, kStripDone);
   }
 }
 
@@ -1180,9 +1099,7 @@ cudaError_t launch_sdtw(int precision, int cells_per_thread, int warps_per_cta, 
                         const SdtwParams &p, const CUtensorMap *tmap, cudaStream_t s) {
   if (p.ref_del) {
     // the anti-diagonal kernels of refdel.cu
-    if (precision == 1) return launch_refdel_fp32(cells_per_thread, warps_per_cta, grid, p, s);
-    if (precision == 0) return launch_refdel_pairs(cells_per_thread, warps_per_cta, grid, p, s);
-    return cudaErrorInvalidValue;
+    return launch_refdel(precision, cells_per_thread, warps_per_cta, grid, p, s);
   }
   if (p.narrow_halo) {
     if (p.state_fp16) {
@@ -1212,9 +1129,7 @@ cudaError_t launch_sdtw(int precision, int cells_per_thread, int warps_per_cta, 
 
 int sdtw_ctas_per_sm(int precision, int cells_per_thread, int warps_per_cta, bool ref_del) {
   if (ref_del) {
-    if (precision == 1) return refdel_fp32_ctas_per_sm(cells_per_thread, warps_per_cta);
-    if (precision == 0) return refdel_pairs_ctas_per_sm(cells_per_thread, warps_per_cta);
-    return 0;
+    return refdel_ctas_per_sm(precision, cells_per_thread, warps_per_cta);
   }
   DTWX_DISPATCH(0, 32, occ_inst)(warps_per_cta);
   DTWX_DISPATCH(0, 48, occ_inst)(warps_per_cta);
