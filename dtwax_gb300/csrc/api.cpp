@@ -768,7 +768,7 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
                            reinterpret_cast<const int32_t *>(dm + L.nsamp),
                            is_i16 ? reinterpret_cast<const float *>(dm + L.smul) : nullptr,
                            is_i16 ? reinterpret_cast<const float *>(dm + L.sadd) : nullptr, n_reads,
-                           h->cfg.norm_eps, c.query.as<float>(), st));
+                           w.max_len, h->cfg.norm_eps, c.query.as<float>(), st));
     ++launches;
   }
   void *d_out = out_dev ? static_cast<void *>(out_dev) : c.results.p;
@@ -1226,7 +1226,7 @@ int dtwx_normalize(dtwx_handle *h, const float *d_raw, const int64_t *offsets, i
   const char *dm = c.meta.as<char>();
   CK(h, launch_normalize(d_raw, 0, reinterpret_cast<const int64_t *>(dm + L.src_off),
                          reinterpret_cast<const int64_t *>(dm + L.dst_off),
-                         reinterpret_cast<const int32_t *>(dm + L.nsamp), nullptr, nullptr, n_reads, h->cfg.norm_eps,
+                         reinterpret_cast<const int32_t *>(dm + L.nsamp), nullptr, nullptr, n_reads, w.max_len, h->cfg.norm_eps,
                          d_query, st));
   h->last_launches = 1;
   return DTWX_OK;
@@ -1649,7 +1649,7 @@ int dtwx_serve_step(dtwx_handle *h) {
   int launches = 0;
   CK(h, launch_normalize(c.raw.p, 0, reinterpret_cast<const int64_t *>(dm + L.src_off),
                          reinterpret_cast<const int64_t *>(dm + L.dst_off),
-                         reinterpret_cast<const int32_t *>(dm + L.nsamp), nullptr, nullptr, nb, h->cfg.norm_eps,
+                         reinterpret_cast<const int32_t *>(dm + L.nsamp), nullptr, nullptr, nb, max_len, h->cfg.norm_eps,
                          c.query.as<float>(), st));
   ++launches;
   double mean = (double)total / nb;

@@ -164,11 +164,11 @@ size_t build_reference_work_bytes(int64_t m);
 
 // Window + z-score of raw reads into the query buffer.
 // src: raw samples (float or int16 when is_i16); for read r the window starts at
-// src_off[r] and has dst_len[r] samples written to dst + dst_off[r].
+// src_off[r] and has dst_len[r] (at most max_len) samples written to dst + dst_off[r].
 cudaError_t launch_normalize(const void *src, int is_i16, const int64_t *src_off,
                              const int64_t *dst_off, const int32_t *dst_len,
                              const float *scale_mul, const float *scale_add, int n_reads,
-                             float eps, float *dst, cudaStream_t s);
+                             int max_len, float eps, float *dst, cudaStream_t s);
 
 // Keys -> dtwx_result records.  When the device error word `err` (may be
 // NULL) is non-zero, every record of the call is marked call =

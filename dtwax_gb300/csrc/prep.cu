@@ -203,17 +203,69 @@ cudaError_t launch_build_reference(const char *d_seq, int64_t L, const double *d
 
 // ---------------------------------------------------------------- normaliser
 // Per read: y = (x - mean) / sqrt(var + eps) over the window, population
-// variance, statistics in FP64, two passes (src/include/normalizer.cu:370-413
-// uses cuDNN batch norm in SPATIAL mode with eps 1e-4 for the same formula).
-// int16 input is first scaled to pA: (raw + add) * mul.
+// variance, two passes (src/include/normalizer.cu:370-413 uses cuDNN batch norm
+// in SPATIAL mode with eps 1e-4 for the same formula).  int16 input is first
+// scaled to pA: (raw + add) * mul.
+//
+// 64-bit accuracy without the FP64 pipe, which has 1/64 of the FP32 rate here
+// (2,048 reads of 1,000 to 8,000 samples, one dtwx_normalize call after the
+// other: 244 us with FP64 passes, 48 now, which is the call's host side and
+// copy; 11 us for the bytes): sums, deviations and products are unevaluated pairs of floats
+// (error-free sums and FMA products, Knuth and Dekker), about 48 bits, and
+// the mean, variance and reciprocal of a read are FP64 in one thread.  The
+// result is the FP64 value rounded to FP32 except where that lies within 2^-47
+// of a rounding boundary.  Reads with samples of 2^40 or more, none above 2^-40,
+// NaN or infinity, or a deviation whose squares leave the FP32 range take the
+// FP64 passes.  The samples of a read are read once and kept in shared memory
+// (up to kNormStaged of them).
+
+constexpr int kNormStaged = 11776;  // 46 KB: with the reductions within the 48 KB that need no opt-in
+
+// s + e == a + b exactly, s the rounded sum.
+__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
+  s = __fadd_rn(a, b);
+  const float bb = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+
+// x - (m0 + m1 + m2) as a pair, |e| about half a unit of d.  (The mean in three
+// parts: two lose bits where the samples lie far from zero for their spread.)
+__device__ __forceinline__ void deviation(float x, float m0, float m1, float m2, float &d, float &e) {
+  float a, b;
+  two_sum(x, -m0, a, b);
+  two_sum(a, -m1, d, e);
+  e += b - m2;
+}
+
+// A sum as an unevaluated pair.
+struct PairSum {
+  float h = 0.f, l = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    float e;
+    two_sum(h, x, h, e);
+    l += e;
+  }
+  __device__ __forceinline__ void warp_reduce() {
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) {
+      const float oh = __shfl_xor_sync(0xffffffffu, h, m), ol = __shfl_xor_sync(0xffffffffu, l, m);
+      add(oh);
+      l += ol;
+    }
+  }
+  __device__ __forceinline__ double value() const { return (double)h + (double)l; }
+};
 
 template <typename T>
 __global__ void __launch_bounds__(kBlock) normalize_kernel(const T *src, const int64_t *src_off,
                                                            const int64_t *dst_off, const int32_t *dst_len,
                                                            const float *scale_mul,
                                                            const float *scale_add, float eps,
-                                                           float *dst) {
+                                                           float *dst, int staged) {
+  extern __shared__ float stage[];
   __shared__ double sh[33];
+  __shared__ uint32_t sh_max[kBlock / 32];
+  __shared__ float sh_part[3];
   const int r = blockIdx.x;
   const int n = dst_len[r];
   if (n <= 0) return;
@@ -221,33 +273,109 @@ __global__ void __launch_bounds__(kBlock) normalize_kernel(const T *src, const i
   float *y = dst + dst_off[r];
   const float mul = scale_mul ? scale_mul[r] : 1.f;
   const float add = scale_add ? scale_add[r] : 0.f;
-  double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += (double)(((float)x[i] + add) * mul);
-  const double mean = block_sum(s, sh) / (double)n;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const auto sample = [&](int i) { return ((float)x[i] + add) * mul; };
+  const bool keep = n <= staged;
+  const auto get = [&](int i) { return keep ? stage[i] : sample(i); };
+
+  // pass 1: sum, and the largest magnitude (NaN and infinity above all others)
+  PairSum s;
+  uint32_t top = 0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += kBlock) {
+    const float v = sample(i);
+    if (keep) stage[i] = v;
+    top = max(top, __float_as_uint(v) & 0x7fffffffu);
+    s.add(v);
+  }
+  s.warp_reduce();
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) {
+    sh[warp] = s.value();
+    sh_max[warp] = top;
+  }
+  __syncthreads();
+  top = 0;
+  for (int i = 0; i < kBlock / 32; ++i) top = max(top, sh_max[i]);
+  constexpr uint32_t kBig = (127u + 40u) << 23, kSmall = (127u - 40u) << 23;
+  bool wild = top >= kBig || top < kSmall;
+  if (!wild) {
+    double mean = 0.0;  // of thread 0
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < kBlock / 32; ++i) mean += sh[i];
+      mean /= (double)n;
+      sh_part[0] = (float)mean;
+      mean -= (double)sh_part[0];
+      sh_part[1] = (float)mean;
+      sh_part[2] = (float)(mean - (double)sh_part[1]);
+    }
+    __syncthreads();
+    const float m0 = sh_part[0], m1 = sh_part[1], m2 = sh_part[2];
+
+    // pass 2: squared deviations
+    PairSum q;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += kBlock) {
+      float d, e;
+      deviation(get(i), m0, m1, m2, d, e);
+      const float p = __fmul_rn(d, d);
+      q.add(p);
+      q.l += fmaf(2.f * d, e, fmaf(d, d, -p));
+    }
+    q.warp_reduce();
+    if (lane == 0) sh[warp] = q.value();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double var = 0.0;
+      for (int i = 0; i < kBlock / 32; ++i) var += sh[i];
+      var /= (double)n;
+      const double inv = 1.0 / sqrt(var + (double)eps);
+      sh_part[0] = (float)inv;
+      sh_part[1] = (float)(inv - (double)(float)inv);
+      sh[32] = var;
+    }
+    __syncthreads();
+    const float ih = sh_part[0], il = sh_part[1];
+    // squares below the FP32 range (a deviation of 2^-60 and less next to no eps)
+    wild = sh[32] < 0x1p-80 && eps < 0x1p-60f;
+    if (!wild) {
+#pragma unroll 4
+      for (int i = threadIdx.x; i < n; i += kBlock) {
+        float d, e;
+        deviation(get(i), m0, m1, m2, d, e);
+        const float p = __fmul_rn(d, ih);
+        y[i] = p + fmaf(e, ih, fmaf(d, il, fmaf(d, ih, -p)));
+      }
+      return;
+    }
+  }
+  __syncthreads();
+  double sd = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) sd += (double)get(i);
+  const double mean = block_sum(sd, sh) / (double)n;
   double q = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double d = (double)(((float)x[i] + add) * mul) - mean;
+    const double d = (double)get(i) - mean;
     q += d * d;
   }
   const double var = block_sum(q, sh) / (double)n;
   const double inv = 1.0 / sqrt(var + (double)eps);
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
-    y[i] = (float)(((double)(((float)x[i] + add) * mul) - mean) * inv);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = (float)(((double)get(i) - mean) * inv);
 }
 
 cudaError_t launch_normalize(const void *src, int is_i16, const int64_t *src_off,
                              const int64_t *dst_off, const int32_t *dst_len, const float *scale_mul,
-                             const float *scale_add, int n_reads, float eps, float *dst,
+                             const float *scale_add, int n_reads, int max_len, float eps, float *dst,
                              cudaStream_t s) {
   if (n_reads <= 0) return cudaSuccess;
+  const int staged = max_len <= kNormStaged ? max_len : kNormStaged;
+  const size_t smem = sizeof(float) * (size_t)(staged > 0 ? staged : 1);
   if (is_i16)
-    normalize_kernel<int16_t><<<n_reads, kBlock, 0, s>>>(static_cast<const int16_t *>(src), src_off,
-                                                         dst_off, dst_len, scale_mul, scale_add, eps,
-                                                         dst);
+    normalize_kernel<int16_t><<<n_reads, kBlock, smem, s>>>(static_cast<const int16_t *>(src), src_off, dst_off,
+                                                            dst_len, scale_mul, scale_add, eps, dst, staged);
   else
-    normalize_kernel<float><<<n_reads, kBlock, 0, s>>>(static_cast<const float *>(src), src_off,
-                                                       dst_off, dst_len, scale_mul, scale_add, eps,
-                                                       dst);
+    normalize_kernel<float><<<n_reads, kBlock, smem, s>>>(static_cast<const float *>(src), src_off, dst_off, dst_len,
+                                                          scale_mul, scale_add, eps, dst, staged);
   return cudaGetLastError();
 }
 
