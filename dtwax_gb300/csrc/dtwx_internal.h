@@ -74,7 +74,8 @@ struct SdtwParams {
   const void *ref_plain;       // reference in global memory (used when TMA is off)
   int64_t m;                   // valid columns per strand
   int64_t m_pad;               // padded columns (multiple of the strip width)
-  int64_t seam_stride;         // bytes of scratch per warp
+  int64_t seam_stride;         // bytes of scratch per warp (two seam columns)
+  int32_t seam_buffers;        // seam columns per CTA: 0 = two per warp; at least one more than its warps
   int32_t n_tasks;
   int32_t n_chunks;            // chunks per task
   int32_t chunk_strips;        // strips per chunk

@@ -34,6 +34,8 @@
 // mixed-precision FMA d*d + min(...) with f16 d and an f32 addend and result.
 #include "dtwx_internal.h"
 
+#include <algorithm>
+#include <atomic>
 #include <cuda/std/cstdint>
 
 #include "team.cuh"
@@ -293,13 +295,16 @@ __device__ __forceinline__ void regs_from_global(const void *base, int lane, RV 
   }
 }
 
-// FP32 strand `strand` out of interleaved (fwd, rev) float pairs.
+// FP32 strand `strand` out of interleaved (fwd, rev) float pairs, of which
+// `cols` (even) may be read; columns past them are past the reference too.
 template <int S>
-__device__ __forceinline__ void regs_from_pairs(const float2 *pairs, int64_t x, int lane, int strand, float (&R)[S]) {
-  const float4 *g = reinterpret_cast<const float4 *>(pairs + x + (int64_t)lane * S);
+__device__ __forceinline__ void regs_from_pairs(const float2 *pairs, int64_t x, int64_t cols, int lane, int strand,
+                                                float (&R)[S]) {
+  const int64_t c0 = x + (int64_t)lane * S;
+  const float4 *g = reinterpret_cast<const float4 *>(pairs + c0);
 #pragma unroll
   for (int k = 0; k < S; k += 2) {
-    const float4 v = __ldg(g + k / 2);
+    const float4 v = c0 + k < cols ? __ldg(g + k / 2) : make_float4(0.f, 0.f, 0.f, 0.f);
     R[k] = strand ? v.y : v.x;
     R[k + 1] = strand ? v.w : v.z;
   }
@@ -359,11 +364,11 @@ __device__ __forceinline__ void sweep_row(typename Pol<PREC>::V (&D)[S], const t
       D[k] = c.x;
       D[k + 1] = c.y;
     }
-    return;
-  }
+  } else {
 #pragma unroll
-  for (int k = S - 1; k >= 1; --k) D[k] = P::cell(R[k], qq, D[k], D[k - 1]);
-  D[0] = P::cell(R[0], qq, D[0], left);
+    for (int k = S - 1; k >= 1; --k) D[k] = P::cell(R[k], qq, D[k], D[k - 1]);
+    D[0] = P::cell(R[0], qq, D[0], left);
+  }
 }
 
 // The MIXED row: reference columns 2k and 2k+1 of the lane share one half2,
@@ -626,7 +631,7 @@ __device__ __forceinline__ bool sweep_strip(const SdtwParams &p, const Strip &st
     __syncwarp();
   } else if constexpr (PREC == 1) {
     if (p.ref_layout == 0)
-      regs_from_pairs<SC>(reinterpret_cast<const float2 *>(p.ref_plain), st.x, lane, st.strand, R);
+      regs_from_pairs<SC>(reinterpret_cast<const float2 *>(p.ref_plain), st.x, p.m_pad, lane, st.strand, R);
     else
       regs_from_global<NW, RV>(reinterpret_cast<const float *>(p.ref_plain) + ref_plane + st.x, lane, R);
   } else if constexpr (PREC == 2) {
@@ -805,7 +810,7 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
   unsigned char *const team_p = smem + nwarps * (STRIP_BYTES + 16 + 384);
   const uint32_t team = smem_u32(team_p);
   const uint32_t prog = team + kTeamStateBytes;
-  const int nbuf = 2 * nwarps;
+  const int nbuf = p.seam_buffers ? p.seam_buffers : 2 * nwarps;
   uint32_t is31 = lane == kWarp - 1 ? 1u : 0u;
   asm volatile("mov.b32 %0, %0;" : "+r"(is31));  // opaque to the optimiser, like lane0_mask
 
@@ -821,8 +826,8 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
 
   const uint32_t lock_a = team, abort_a = team + 4, item_a = team + 8, next_a = team + 12, total_a = team + 16,
                  seq_a = team + 20, dealt_a = team + 24;
-  char *const seam_base = p.seam + (int64_t)blockIdx.x * nwarps * p.seam_stride;
   const int64_t seam_half = p.seam_stride / 2;
+  char *const seam_base = p.seam + (int64_t)blockIdx.x * nbuf * seam_half;
   // FP32 and MIXED split each (task, chunk) into one work item per strand
   const int nstr = !PAIRS ? (p.strands > 0 ? p.strands : 2) : 1;
   const int per_task = p.n_chunks * nstr;
@@ -1127,7 +1132,7 @@ cudaError_t launch_sdtw(int precision, int cells_per_thread, int warps_per_cta, 
   return cudaErrorInvalidValue;
 }
 
-int sdtw_ctas_per_sm(int precision, int cells_per_thread, int warps_per_cta, bool ref_del) {
+static int query_ctas_per_sm(int precision, int cells_per_thread, int warps_per_cta, bool ref_del) {
   if (ref_del) {
     return refdel_ctas_per_sm(precision, cells_per_thread, warps_per_cta);
   }
@@ -1140,6 +1145,23 @@ int sdtw_ctas_per_sm(int precision, int cells_per_thread, int warps_per_cta, boo
   DTWX_DISPATCH(2, 48, occ_inst)(warps_per_cta);
   DTWX_DISPATCH(2, 64, occ_inst)(warps_per_cta);
   return 0;
+}
+
+// A property of the compiled instance on this GPU model, asked several times
+// per call while a shape is picked: the occupancy API is asked once.
+int sdtw_ctas_per_sm(int precision, int cells_per_thread, int warps_per_cta, bool ref_del) {
+  static std::atomic<int8_t> known[2][3][5][17];  // 0: not asked yet, else 1 + CTAs
+  const int c = cells_per_thread / 16;
+  if (precision < 0 || precision > 2 || c < 1 || c > 4 || cells_per_thread != 16 * c || warps_per_cta < 1 ||
+      warps_per_cta > 16)
+    return 0;
+  std::atomic<int8_t> &k = known[ref_del ? 1 : 0][precision][c][warps_per_cta];
+  int8_t v = k.load(std::memory_order_relaxed);
+  if (v == 0) {
+    v = (int8_t)(1 + std::min(query_ctas_per_sm(precision, cells_per_thread, warps_per_cta, ref_del), 100));
+    if (v > 1) k.store(v, std::memory_order_relaxed);  // (an error is asked again)
+  }
+  return v - 1;
 }
 
 // ---------------------------------------------------------------- issue-rate probe

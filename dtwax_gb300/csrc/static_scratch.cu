@@ -10,10 +10,12 @@
 // scratch the sweep needs (task table, work counter, per-warp seam columns,
 // per-read result keys) lives in the fixed array below, which the library
 // reserves once when it is loaded onto a GPU and keeps until the process exits.
+#include <algorithm>
 #include <mutex>
 
 #include "dtwx.h"
 #include "dtwx_internal.h"
+#include "sweep_shape.h"
 
 namespace dtwx {
 namespace {
@@ -21,28 +23,26 @@ namespace {
 // Limits of the static scratch.
 constexpr int kStMaxReads = 4096;   // reads per call
 constexpr int kStMaxRows = 2048;    // samples per read (QUERY_LEN of the reference)
-constexpr int kStCells = 16;        // FP32 instance: 16 column pairs per lane (512-column strips)
-constexpr int kStWarps = 4;         // warps per CTA
-constexpr int kStCtas = 64;         // CTAs: 256 warps share the queue
-constexpr int kStPairBytes = 8;     // float2 (fwd, rev)
+constexpr int kStCells = 48;        // FP32 instance: 48 columns per lane (1,536-column strips)
+constexpr int kStWarps = 4;         // warps per CTA: a team that sweeps an item's strips together
+constexpr int kStBuffers = kStWarps + 1;  // seam columns of a CTA, the fewest a team works with
+constexpr int kStColAlign = 512;    // columns up to whose next multiple the caller's reference is readable
 
 constexpr int64_t align256(int64_t x) { return (x + 255) & ~(int64_t)255; }
-// seam scratch of one warp: the kernel's own layout (seam_bytes_per_warp, with
-// its slack for whole-warp stores past the last row) for the widest seam entry
-// the FP32 sweep could use, so that a change of the cell size or the slack
-// cannot let a warp write past the array
-constexpr int64_t kStSeamPerWarp = seam_bytes_per_warp(kStPairBytes, kStMaxRows);
-static_assert(kStPairBytes >= 4, "FP32 seam cells are 4 bytes");
-static_assert(kStSeamPerWarp % 256 == 0, "per-warp seam scratch keeps 256-byte alignment");
+// bytes of one seam column of `rows` rows: FP32 cells, the row above the first
+// and 32 entries of slack for whole-warp stores past the last
+constexpr int64_t st_column_bytes(int rows) { return align256((int64_t)(rows + 1 + 32) * 4); }
+// Seam columns: 9 MB, which the CTAs of a call share out by the rows of its
+// longest read: 214 CTAs at 2,048 rows, all that fit on the GPU below about 950.
+constexpr int64_t kStSeamBytes = 9043968;
 
 constexpr int64_t kStFlagsOff = 0;                                                // counter, error flags
 constexpr int64_t kStKeysOff = 256;                                               // 2 x u64 per read
 constexpr int64_t kStTasksOff = align256(kStKeysOff + 16 * (int64_t)kStMaxReads);  // Task per read
 constexpr int64_t kStNsampOff = align256(kStTasksOff + 32 * (int64_t)kStMaxReads); // int32 per read
 constexpr int64_t kStSeamOff = align256(kStNsampOff + 4 * (int64_t)kStMaxReads);
-constexpr int64_t kStBytes = kStSeamOff + kStSeamPerWarp * kStWarps * kStCtas;     // about 9 MiB
-static_assert(kStSeamOff + seam_bytes_per_warp(4, kStMaxRows) * kStWarps * kStCtas <= kStBytes,
-              "every warp's seam columns fit in the static scratch");
+constexpr int64_t kStBytes = kStSeamOff + kStSeamBytes;     // about 9 MiB
+static_assert(kStSeamBytes >= 152 * kStBuffers * st_column_bytes(kStMaxRows), "a CTA on every SM at the row limit");
 
 // The scratch itself.  Host code must never pass this name to a kernel: on the
 // host it is only a stand-in symbol, not a device address.  The device address
@@ -102,7 +102,8 @@ extern "C" int dtwx_distances_static(const void *d_ref_pairs, int64_t ref_len, c
   // Host-side task table in a fixed host array (no allocation either).
   static thread_local Task h_tasks[kStMaxReads];
   static thread_local int32_t h_nsamp[kStMaxReads];
-  int32_t n_tasks = 0;
+  int32_t n_tasks = 0, max_rows = 0;
+  int64_t sum_rows = 0;
   for (int r = 0; r < n_reads; ++r) {
     const int64_t n = offsets[r + 1] - offsets[r];
     if (n < 0) return st_fail(DTWX_E_ARG, "dtwx_distances_static: offsets must be non-decreasing");
@@ -117,6 +118,8 @@ extern "C" int dtwx_distances_static(const void *d_ref_pairs, int64_t ref_len, c
     t.state_off = 0;
     t.out_slot = r;
     t.pad = 0;
+    max_rows = std::max(max_rows, (int32_t)n);
+    sum_rows += n;
   }
   if (n_reads == 0) return DTWX_OK;
 
@@ -148,21 +151,41 @@ extern "C" int dtwx_distances_static(const void *d_ref_pairs, int64_t ref_len, c
     p.err = flags + 4;
     p.ref_plain = d_ref_pairs;
     p.m = ref_len;
-    p.m_pad = ref_len;
-    p.seam_stride = kStSeamPerWarp;
+    p.m_pad = (ref_len + kStColAlign - 1) / kStColAlign * kStColAlign;  // readable columns
+    const int64_t column = st_column_bytes(max_rows);
+    p.seam_stride = 2 * column;
+    p.seam_buffers = kStBuffers;
     p.n_tasks = n_tasks;
+    // teams: what the scratch holds and the GPU has room for; chunks: the widest
+    // of the fastest by the estimate (any chunk width gives the same bits)
+    int sms = 0, occ = sdtw_ctas_per_sm(1, kStCells, kStWarps);
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+      return st_fail(DTWX_E_CUDA, cudaGetErrorString(e));
+    const int64_t teams =
+        std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * std::max(occ, 1), kStSeamBytes / (kStBuffers * column)));
     const int64_t W = (int64_t)kWarp * kStCells;
     const int64_t strips = (ref_len + W - 1) / W;
-    // one chunk of G strips per item: about 4 items per warp for the whole batch
-    int64_t g = (strips * n_tasks + 4LL * kStWarps * kStCtas - 1) / (4LL * kStWarps * kStCtas);
-    if (g < 1) g = 1;
-    if (g > strips) g = strips;
-    p.chunk_strips = (int32_t)g;
-    p.n_chunks = (int32_t)((strips + g - 1) / g);
-    p.max_rows = kStMaxRows;
+    const double rows = (double)sum_rows / n_tasks;
+    double best = 1e300;
+    int64_t g_best = strips, chunks = 0;
+    for (int64_t g = 1; g <= strips; g = chunks > 1 ? (strips + chunks - 2) / (chunks - 1) : g + 1) {
+      chunks = (strips + g - 1) / g;
+      const double halo = chunks > 1 ? (rows + W) / (2.0 * W) * (double)(chunks - 1) / (double)chunks : 0.0;
+      const double t = sweep_estimate(kRowCost[1][2], 2 * n_tasks * chunks, (double)g + halo,
+                                      (double)g + (chunks > 1 ? std::ceil(rows / W) : 0.0), rows, kStWarps, teams, sms);
+      if (t < best) {
+        best = t;
+        g_best = g;
+      }
+    }
+    p.chunk_strips = (int32_t)g_best;
+    p.n_chunks = (int32_t)((strips + g_best - 1) / g_best);
+    p.max_rows = max_rows;
     p.n_items = (int32_t)((int64_t)n_tasks * p.n_chunks);
+    const int64_t items = 2 * (int64_t)n_tasks * p.n_chunks;
+    const int grid = (int)std::min<int64_t>(teams, items);
     p.use_tma = 0;
-    if ((e = launch_sdtw(1, kStCells, kStWarps, kStCtas, p, nullptr, st)) != cudaSuccess)
+    if ((e = launch_sdtw(1, kStCells, kStWarps, grid, p, nullptr, st)) != cudaSuccess)
       return st_fail(DTWX_E_CUDA, cudaGetErrorString(e));
   }
   if ((e = launch_finalize(keys, d_nsamp, n_reads, 0, ref_len, threshold, flags + 4, d_out, st)) != cudaSuccess)
