@@ -596,9 +596,9 @@ __device__ __forceinline__ bool sweep_strip(const SdtwParams &p, const Strip &st
   constexpr int K = kRescaleRows;
   // rows per group of the window loop, and how their seam cells leave it, by
   // what the instruction schedule measured (64 strips of one read per item,
-  // Tcell/s): FP16 pairs, 4 rows and one 16-byte store 17.8, a store per row
-  // 15.2, 2 rows 15.5; FP32, 4 rows and a store per row 12.9, one 16-byte
-  // store 12.7, 2 rows 12.5; MIXED, 2 rows and a store per row 13.9, 4 rows 13.6
+  // Tcell/s): FP16 pairs, 4 rows and one 16-byte store 18.1, a store per row
+  // 15.2, 2 rows 15.8; FP32, 4 rows and a store per row 12.9, one 16-byte
+  // store 12.6, 2 rows 12.6; MIXED, 2 rows and a store per row 13.4, 4 rows 12.9
   constexpr int kRows = PREC == 2 ? 2 : 4;
   const int n = st.n, rows = st.rows;
   const bool first = st.first;
@@ -668,15 +668,13 @@ __device__ __forceinline__ bool sweep_strip(const SdtwParams &p, const Strip &st
     st_shared_u32(wb + 4u * (uint32_t)lane, qb);
     st_shared_u32(wb + 128u + 4u * (uint32_t)lane, cell_bits<PREC>(swin));
     __syncwarp();
-    // the next window's samples, and its seam values from the left neighbour's
-    // next window.  FP32 and MIXED cells fetch what is complete ahead of this
-    // window's rows; FP16 pairs fetch it all after them (the registers that
-    // would hold it cost the rows more: 17.8 against 18.2 Tcell/s)
+    // the next window's seam values come from the left neighbour's next window.
+    // FP32 cells fetch them ahead of this window's rows if it is complete by now;
+    // FP16 and MIXED fetch them after the rows (the registers that would hold them
+    // cost the rows more: 16.8 against 18.1 and 12.6 against 13.4 Tcell/s)
     const int r = i0 + kWarp + lane;
     const bool more = !first && i0 + kWarp < rows;
-    const bool ahead = PREC != 0 && more && team_ready(st.prog_in, tag_in | (win + 2));
-    float qn = 0.f;
-    if constexpr (PREC == 2) qn = r < n ? q[r] : 0.f;
+    const bool ahead = PREC == 1 && more && team_ready(st.prog_in, tag_in | (win + 2));
     V sn = vinf;
     float2 off_next = O;
     if (ahead && r < rows) sn = seam_in[r];
@@ -744,6 +742,10 @@ __device__ __forceinline__ bool sweep_strip(const SdtwParams &p, const Strip &st
       so[lane] = lane < cnt ? P::from_bits(ld_shared_u32(wb + 256u + 4u * (uint32_t)lane)) : vinf;
     }
     so += kWarp;
+    // (the samples' load goes out before the publish for FP16 pairs, 3 % on narrow
+    // chunks, and after it for the others, 4 % on FP32)
+    float qn = 0.f;
+    if constexpr (PREC == 0) qn = r < n ? q[r] : 0.f;
     ++win;
     team_publish(st.prog_out, st.seq, win);
     if (more && !ahead) {
@@ -751,7 +753,7 @@ __device__ __forceinline__ bool sweep_strip(const SdtwParams &p, const Strip &st
       if (r < rows) sn = seam_in[r];
       if constexpr (PREC == 0) off_next = off_in[win];
     }
-    if constexpr (PREC != 2) qn = r < n ? q[r] : 0.f;
+    if constexpr (PREC != 0) qn = r < n ? q[r] : 0.f;
     qb = qw_bits<PREC>(qn);
     swin = sn;
     if constexpr (PREC == 0) {
