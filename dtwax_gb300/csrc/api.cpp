@@ -928,11 +928,11 @@ int create_common(const dtwx_config *cfg_in, const std::vector<double> &table, c
   DevBuf d_seq, d_table, d_work;
   if ((e = d_seq.ensure(L)) != cudaSuccess) return bad(e, "alloc seq");
   if ((e = d_table.ensure(sizeof(double) * kTableSize)) != cudaSuccess) return bad(e, "alloc table");
-  if ((e = d_work.ensure(build_reference_work_bytes(m))) != cudaSuccess) return bad(e, "alloc work");
+  if ((e = d_work.ensure(build_reference_work_bytes())) != cudaSuccess) return bad(e, "alloc work");
   cudaMemcpyAsync(d_seq.p, seq.data(), L, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(d_table.p, table.data(), sizeof(double) * kTableSize, cudaMemcpyHostToDevice, st);
   e = launch_build_reference(d_seq.as<char>(), L, d_table.as<double>(), m, h->m_pad,
-                             cfg.strand_mode == DTWX_STRANDS_CONCAT, d_work.as<double>(), h->ref16.as<__half2>(),
+                             cfg.strand_mode == DTWX_STRANDS_CONCAT, d_work.p, h->ref16.as<__half2>(),
                              h->ref32.as<float>(), h->ref16p.as<__half>(), h->fwd32.as<float>(),
                              h->rev32.as<float>(), st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1057,6 +1057,7 @@ int dtwx_destroy(dtwx_handle *h) {
   if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
   h->ref16.release();
   h->ref32.release();
+  h->ref16p.release();
   h->fwd32.release();
   h->rev32.release();
   h->state.release();

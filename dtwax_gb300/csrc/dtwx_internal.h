@@ -158,10 +158,10 @@ int sdtw_ref_bytes(int precision);   // reference bytes per column of a strip
 // Reference builder: genome bytes -> z-scored levels as FP16 (fwd, rev) pairs,
 // as FP32 planes (fwd plane, then rev plane at m_pad) and as FP16 planes.
 cudaError_t launch_build_reference(const char *d_seq, int64_t L, const double *d_table,
-                                   int64_t m, int64_t m_pad, int concat, double *d_work,
+                                   int64_t m, int64_t m_pad, int concat, void *d_work,
                                    __half2 *d_ref16, float *d_ref32, __half *d_ref16p, float *d_fwd32,
                                    float *d_rev32, cudaStream_t s);
-size_t build_reference_work_bytes(int64_t m);
+size_t build_reference_work_bytes();
 
 // Window + z-score of raw reads into the query buffer.
 // src: raw samples (float or int16 when is_i16); for read r the window starts at

