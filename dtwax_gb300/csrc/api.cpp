@@ -549,10 +549,15 @@ int enqueue_sweep(dtwx_handle *h, BatchCtx &c, int precision, cudaStream_t st, c
   return DTWX_OK;
 }
 
-int check_device_flags(dtwx_handle *h, BatchCtx &c) {
+// The status of the device error word.  `copied`: the word is on its way to
+// c.h_flags with work that has been waited for; else it is fetched here.
+int check_device_flags(dtwx_handle *h, BatchCtx &c, bool copied = false) {
   int32_t f[8] = {0};
   if (!c.flags.p) return DTWX_OK;
-  CK(h, cudaMemcpy(f, c.flags.p, sizeof(f), cudaMemcpyDeviceToHost));
+  if (copied)
+    memcpy(f, c.h_flags.p, sizeof(f));
+  else
+    CK(h, cudaMemcpy(f, c.flags.p, sizeof(f), cudaMemcpyDeviceToHost));
   if (f[4]) CK(h, cudaMemset(c.flags.as<int32_t>() + 4, 0, sizeof(int32_t)));  // reported once
   if (f[4] & kErrTmaTimeout) return fail(h, DTWX_E_TIMEOUT, "device: TMA wait gave up");
   if (f[4] & kErrBadTask) return fail(h, DTWX_E_CAPACITY, "device: task longer than the seam buffers");
@@ -831,11 +836,17 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
     c.meta_pending = true;
   }
   if (out_host) {
-    if (n_reads)
-      CK(h, cudaMemcpyAsync(out_host, d_out, sizeof(dtwx_result) * (size_t)n_reads, cudaMemcpyDeviceToHost, st));
+    // results and error word into pinned memory, one wait for both (a pageable
+    // copy and a second round trip for the word cost a call of 10 reads 10 us of 460)
+    const size_t bytes = sizeof(dtwx_result) * (size_t)n_reads;
+    CK(h, c.h_results.ensure(std::max<size_t>(bytes, 16)));
+    CK(h, c.h_flags.ensure(64));
+    if (n_reads) CK(h, cudaMemcpyAsync(c.h_results.p, d_out, bytes, cudaMemcpyDeviceToHost, st));
+    if (c.flags.p) CK(h, cudaMemcpyAsync(c.h_flags.p, c.flags.p, 64, cudaMemcpyDeviceToHost, st));
     CK(h, cudaStreamSynchronize(st));
     c.meta_pending = false;
-    if (int rc = check_device_flags(h, c)) return rc;
+    if (n_reads) memcpy(out_host, c.h_results.p, bytes);
+    if (int rc = check_device_flags(h, c, true)) return rc;
   } else {
     // device results: the error word is read by dtwx_sync (and marked in the results)
     CK(h, cudaEventRecord(c.done, st));
