@@ -49,6 +49,7 @@ import os
 import subprocess
 
 import numpy as np
+import unittest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT_DIR = os.path.join(HERE, "_ref")
@@ -179,6 +180,11 @@ def tile_interleave(cols: np.ndarray, tiles: int) -> np.ndarray:
     return out
 
 
+class CubinMissing(FileNotFoundError, unittest.SkipTest):
+    """A cubin that could not be built here; a test that needs it is skipped,
+    from a fixture too."""
+
+
 class RefKernel:
     """One reference-kernel geometry loaded on the current CUDA device."""
 
@@ -187,7 +193,7 @@ class RefKernel:
         if name not in GEOMETRIES:
             raise KeyError(name)
         if not available(name):
-            raise FileNotFoundError(f"{cubin_path(name)} not built (needs the reference's sources at build time)")
+            raise CubinMissing(f"{cubin_path(name)} not built (needs the reference's sources at build time)")
         self.name = name
         self.precision, self.ref_len, self.ref_del = GEOMETRIES[name]
         self.tiles = self.ref_len // TILE
