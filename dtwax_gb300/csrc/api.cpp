@@ -317,28 +317,40 @@ int default_team(int precision, int full, double mean_rows, int64_t items, int G
 
 // Which warp of a CTA takes the p-th strip of a dealt batch's first round
 // (4 bits per strip): heavy strips (the chunk's own, S cells per lane) and
-// narrow halo strips spread evenly over the SM's four schedulers (warp w runs
-// on scheduler w mod 4), largest first.
-uint64_t deal_warps(int warps, int nh, int g, int S, int SH, double rows, int WH) {
+// narrow halo strips spread over the SM's four schedulers (warp w runs on
+// scheduler w mod 4) by what a row of each costs, the longer first among
+// equals.  By rows, not by a strip's whole work: the strips of an item run in
+// step, each behind its left neighbour, so a scheduler that holds four halo
+// strips slows down the own strip they feed, however short they are
+// (9 reads of 2,048 samples against 48 kb: 398 us by work, 357 by rows; one
+// read: 392 and 275).
+uint64_t deal_warps(int warps, int64_t strips, int nh, int g, int S, int SH, double rows, int WH) {
+  const int placed = (int)std::min<int64_t>(warps, strips), per = nh + g;
   double weight[16], load[4] = {0, 0, 0, 0};
   int order[16], used[4] = {0, 0, 0, 0};
-  const int per = nh + g;
-  for (int p = 0; p < warps; ++p) {
+  for (int p = 0; p < placed; ++p) {
     const int s = p % per;
-    // rows of halo strip s: those that still reach the chunk
-    const double r = s < nh ? std::max(1.0, std::min(rows, rows - (double)s * WH)) : rows;
-    weight[p] = r * (s < nh ? SH : S);
+    const double length = s < nh ? std::max(1.0, rows - (double)s * WH) : rows;
+    // (3: the row's shuffle, loads and loop; the last halo strip feeds the chunk
+    // and gets the most room of its kind)
+    weight[p] = (s < nh ? SH : S) + 3.0 + 1e-3 * length / rows + (s == nh - 1 ? 1.0 : 0.0);
     order[p] = p;
   }
-  std::stable_sort(order, order + warps, [&](int a, int b) { return weight[a] > weight[b]; });
-  uint64_t map = 0;
-  for (int i = 0; i < warps; ++i) {
+  std::stable_sort(order, order + placed, [&](int a, int b) { return weight[a] > weight[b]; });
+  uint64_t map = 0, taken = 0;
+  for (int i = 0; i < placed; ++i) {
     const int p = order[i];
     int best = -1;
     for (int q = 0; q < 4; ++q)
       if (4 * used[q] + q < warps && (best < 0 || load[q] < load[best])) best = q;
     load[best] += weight[p];
-    map |= (uint64_t)(4 * used[best]++ + best) << (4 * p);
+    const int w = 4 * used[best]++ + best;
+    map |= (uint64_t)w << (4 * p);
+    taken |= 1ull << w;
+  }
+  for (int p = placed, w = 0; p < warps; ++p, ++w) {  // (warps without a strip of the first round)
+    while (taken >> w & 1) ++w;
+    map |= (uint64_t)w << (4 * p);
   }
   return map;
 }
@@ -436,7 +448,7 @@ Shape pick_shape(dtwx_handle *h, int precision, int64_t n_tasks, double mean_row
     // a batch whose strips can all run at once: one CTA per SM, its items dealt
     // out in turn (first come, first served, the CTAs that start first take more
     // than their share) and its strips placed by weight.  (10 reads of 2,048
-    // samples against 48 kb: 0.39 ms, 0.52 without.)  Batches of very short reads
+    // samples against 48 kb: 0.45 ms, 0.52 without.)  Batches of very short reads
     // are over before the first round's bookkeeping pays
     const int64_t strips_all = s.items * ((int64_t)s.G + nh);
     if ((precision != 0 || s.nh) && full <= 16 && strips_all <= (int64_t)h->sms * full * 3 / 2 &&
@@ -444,7 +456,8 @@ Shape pick_shape(dtwx_handle *h, int precision, int64_t n_tasks, double mean_row
       s.deal = true;
       s.warps = full;
       occ = 1;
-      s.deal_warps = deal_warps(full, nh, s.G, s.S, SH, mean_rows, kWarp * SH);
+      s.deal_warps = deal_warps(full, (s.items + h->sms - 1) / h->sms * ((int64_t)s.G + nh), nh, s.G, s.S, SH,
+                                mean_rows, kWarp * SH);
     } else if (precision == 0 || mean_rows < 384) {
       const int k = default_team(precision, full, mean_rows, s.items, s.G, h->sms);
       if (k != s.warps && sdtw_ctas_per_sm(precision, s.S, k, false) >= 1) {
