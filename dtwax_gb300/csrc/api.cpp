@@ -819,9 +819,6 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
       p.team_warps = sh.team;
       p.deal = sh.deal ? 1 : 0;
       p.deal_warps = sh.deal_warps;
-    p.team_warps = sh.team;
-    p.deal = sh.deal ? 1 : 0;
-    p.deal_warps = sh.deal_warps;
         const int ii = inst_index(precision, sh.S);
       p.use_tma = h->tmap_ok[precision][ii] ? 1 : 0;
       CK(h, launch_sdtw(precision, sh.S, sh.warps, sh.grid, p, p.use_tma ? &h->tmap[precision][ii] : nullptr,
@@ -1295,13 +1292,13 @@ int dtwx_autotune(dtwx_handle *h, int32_t n_reads_req, int32_t read_len, float *
   struct Cand { int S, warps, permille; };
   std::vector<Cand> cands;
   const bool rd = h->cfg.recurrence == DTWX_REF_DEL;
-  // warps 0: the default shape (for REF_DEL the batch spread evenly over the SMs)
+  // warps 0: the default teams (REF_DEL)
   for (int si = 0; si < inst_count(prec); ++si)
     for (int w : {0, 4, 8})
       for (int pm : {500, 1000, 2000}) {
         if (!sdtw_instance_exists(prec, inst_S(prec, si), rd)) continue;
         if (rd && pm != 1000) continue;  // one chunk per task: no chunk width to tune
-        if (w == 0 && !rd) continue;     // the default is 4 warps
+        if (w == 0 && !rd) continue;     // (a tuned NO_REF_DEL shape has CTAs of 4 or 8 warps)
         if (w && !sdtw_ctas_per_sm(prec, inst_S(prec, si), w, rd)) continue;
         cands.push_back({inst_S(prec, si), w, pm});
       }

@@ -13,15 +13,19 @@
 // it from the seam column written by the strip to the left.
 //
 // A work item is (task, chunk): the task's rows against output columns
-// [a, b) of the reference.  The warp sweeps the strips of [x0, b) left to right
-// (ref strip staged into shared memory by a TMA tensor copy, double buffered),
-// handing each strip's last column to the next strip through per-warp
-// scratch.  Chunks are independent: a chunk starting at a > 0 recomputes a
-// halo of >= n columns to its left, with +inf entering at the halo's left edge;
-// that error moves right one column per row, so it never reaches column a.
-// Halo strips stop at the last row that can still influence column a.  In the
-// NH instances they are narrower than the chunk's own strips, so the swept
-// halo follows that shrinking triangle more closely.
+// [a, b) of the reference.  The warps of a CTA form a team (team.cuh): the
+// strips of [x0, b) are handed out left to right, and the warp of strip s + 1
+// runs a window of 32 rows behind the warp of strip s, whose last column
+// reaches it through a seam buffer in global scratch.  An item therefore lasts
+// about as long as its strips divided by the team's warps, not as long as one
+// warp takes for all of them.  Each warp stages its strip's slice of the
+// reference into shared memory by a TMA tensor copy and reads it into
+// registers once per strip.  Chunks are independent: a chunk starting at a > 0
+// recomputes a halo of >= n columns to its left, with +inf entering at the
+// halo's left edge; that error moves right one column per row, so it never
+// reaches column a.  Halo strips stop at the last row that can still influence
+// column a.  In the NH instances they are narrower than the chunk's own
+// strips, so the swept halo follows that shrinking triangle more closely.
 //
 // FP16: cells are __half2 (fwd strand in .x, rev in .y).  Every kRescaleRows
 // rows each strip subtracts its own row minimum from its cells and adds it to

@@ -15,7 +15,8 @@ namespace dtwx {
 // so a strip's left neighbour was always handed out before it, and no warp
 // waits for work that has not begun.  Strip `seq` of a team writes its seam
 // column into buffer seq % buffers (two per warp, or as few as one more than
-// the warps); prog[] of that buffer holds the sequence number and how much of it is complete (32-row windows in sdtw.cu, rows in refdel.cu).
+// the warps); prog[] of that buffer holds the sequence number and how much of
+// it is complete (32-row windows in sdtw.cu, rows in refdel.cu).
 struct TeamState {
   uint32_t lock;
   uint32_t abort;  // a wait of this CTA gave up: every warp leaves
