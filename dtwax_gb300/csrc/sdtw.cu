@@ -864,12 +864,17 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
   // A dealt batch's first round: warp w takes the strip that p.deal_warps
   // gives it, walking the CTA's items to find it; the warp with the last one
   // leaves the cursor behind it.
-  // It waits in the word beside the warp's mbarrier: in registers it lived
-  // through every row (4 reads of 1,600 samples against 5 Mb: 4.26 to 4.22 ms).
+  // FP16 pairs keep it in the word beside the warp's mbarrier: in registers it
+  // lived through every row (4 reads of 1,600 samples against 5 Mb: 4.26 to
+  // 4.22 ms).  FP32 and MIXED keep it in registers, which their schedule
+  // takes better (192 reads of 2,000 samples against 1 Mb: 60.8 and 58.4 ms,
+  // 61.4 and 59.2 through shared memory).
+  constexpr bool FIRST_SHARED = PREC == 0;
   const uint32_t first_a = smem_u32(bar + 1);
-  if constexpr (DEAL) st_shared_u64(first_a, 0);
+  if constexpr (DEAL && FIRST_SHARED) st_shared_u64(first_a, 0);
+  int first_item = -1, first_s = 0;
+  uint32_t first_seq = 0;
   if (DEAL && p.deal) {
-    int first_item, first_s = 0;
     int pos = 0;
     while (pos < 15 && (int)((p.deal_warps >> (4 * pos)) & 15u) != warp) ++pos;
     int at = 0, total = 0, dealt = 0;
@@ -883,6 +888,7 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
     if (item < n_items) {
       first_item = (int)item;
       first_s = pos - at;
+      first_seq = (uint32_t)pos;
     } else {
       first_item = (int)n_items;  // fewer strips than warps
     }
@@ -893,8 +899,8 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
       st_shared_volatile(seq_a, (uint32_t)nwarps);
       st_shared_volatile(dealt_a, (uint32_t)dealt);
     }
-    st_shared_u64(first_a, (uint64_t)(0x80000000u | (uint32_t)pos << 8 | (uint32_t)first_s) << 32 |
-                               (uint32_t)first_item);  // strips of a first round: at most 16
+    if constexpr (FIRST_SHARED)  // (strips of a first round: at most 16)
+      st_shared_u64(first_a, (uint64_t)(0x80000000u | first_seq << 8 | (uint32_t)first_s) << 32 | (uint32_t)first_item);
     __syncthreads();
   }
 
@@ -903,7 +909,10 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
     // lane runs the same instructions (only the atomics are lane 0's).
     int item = -1, s = 0;
     uint32_t seq = 0;
-    if constexpr (DEAL) {
+    if constexpr (DEAL && !FIRST_SHARED) {
+      item = first_item, s = first_s, seq = first_seq;
+      first_item = -1;
+    } else if constexpr (DEAL) {
       const uint64_t f = ld_shared_u64(first_a);
       if (f) {
         item = (int)(uint32_t)f;
