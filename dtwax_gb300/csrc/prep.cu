@@ -216,10 +216,12 @@ cudaError_t launch_build_reference(const char *d_seq, int64_t L, const double *d
 //
 // 64-bit accuracy without the FP64 pipe, which has 1/64 of the FP32 rate here
 // (2,048 reads of 1,000 to 8,000 samples, one dtwx_normalize call after the
-// other: 244 us with FP64 passes, 48 now, which is the call's host side and
-// copy; 11 us for the bytes): sums, deviations and products are unevaluated pairs of floats
+// other: 244 us with FP64 passes, 43 now; 11 us for the bytes): sums, deviations and products are unevaluated pairs of floats
 // (error-free sums and FMA products, Knuth and Dekker), about 48 bits, and
-// the mean, variance and reciprocal of a read are FP64 in one thread.  The
+// the mean, variance and reciprocal root of a read are FP64 in one warp, with as
+// few instructions as they take: a warp's total converted by each warp, added by
+// one thread and divided twice cost 6 us of the 43, and a third of the time of
+// short reads (4,096 of 200 to 400 samples: 47 us, 31 now).  The
 // result is the FP64 value rounded to FP32 except where that lies within 2^-47
 // of a rounding boundary.  Reads with samples of 2^40 or more, none above 2^-40,
 // NaN or infinity, or a deviation whose squares leave the FP32 range take the
@@ -260,8 +262,18 @@ struct PairSum {
       l += ol;
     }
   }
-  __device__ __forceinline__ double value() const { return (double)h + (double)l; }
 };
+
+// Total of the warps' sums, in FP64: `part` holds a pair per warp; every lane of
+// the calling warp gets it.  (Eight lanes convert and add at once: an FP64
+// instruction holds its pipe 16 cycles for one lane as for 32.)
+__device__ __forceinline__ double warps_total(const float2 *part, int lane) {
+  double v = 0.0;
+  if (lane < kBlock / 32) v = (double)part[lane].x + (double)part[lane].y;
+#pragma unroll
+  for (int m = kBlock / 64; m >= 1; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+  return v;
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kBlock) normalize_kernel(const T *src, const int64_t *src_off,
@@ -272,7 +284,8 @@ __global__ void __launch_bounds__(kBlock) normalize_kernel(const T *src, const i
   extern __shared__ float stage[];
   __shared__ double sh[33];
   __shared__ uint32_t sh_max[kBlock / 32];
-  __shared__ float sh_part[3];
+  __shared__ float sh_part[4];
+  __shared__ float2 sh_pair[kBlock / 32];
   const int r = blockIdx.x;
   const int n = dst_len[r];
   if (n <= 0) return;
@@ -284,6 +297,9 @@ __global__ void __launch_bounds__(kBlock) normalize_kernel(const T *src, const i
   const auto sample = [&](int i) { return ((float)x[i] + add) * mul; };
   const bool keep = n <= staged;
   const auto get = [&](int i) { return keep ? stage[i] : sample(i); };
+
+  double rn = 0.0;  // of warp 0, whose division overlaps the loads of the others
+  if (warp == 0) rn = 1.0 / (double)n;
 
   // pass 1: sum, and the largest magnitude (NaN and infinity above all others)
   PairSum s;
@@ -298,7 +314,7 @@ __global__ void __launch_bounds__(kBlock) normalize_kernel(const T *src, const i
   s.warp_reduce();
   top = __reduce_max_sync(0xffffffffu, top);
   if (lane == 0) {
-    sh[warp] = s.value();
+    sh_pair[warp] = make_float2(s.h, s.l);
     sh_max[warp] = top;
   }
   __syncthreads();
@@ -307,14 +323,14 @@ __global__ void __launch_bounds__(kBlock) normalize_kernel(const T *src, const i
   constexpr uint32_t kBig = (127u + 40u) << 23, kSmall = (127u - 40u) << 23;
   bool wild = top >= kBig || top < kSmall;
   if (!wild) {
-    double mean = 0.0;  // of thread 0
-    if (threadIdx.x == 0) {
-      for (int i = 0; i < kBlock / 32; ++i) mean += sh[i];
-      mean /= (double)n;
-      sh_part[0] = (float)mean;
-      mean -= (double)sh_part[0];
-      sh_part[1] = (float)mean;
-      sh_part[2] = (float)(mean - (double)sh_part[1]);
+    if (warp == 0) {
+      double mean = warps_total(sh_pair, lane) * rn;
+      if (lane == 0) {
+        sh_part[0] = (float)mean;
+        mean -= (double)sh_part[0];
+        sh_part[1] = (float)mean;
+        sh_part[2] = (float)(mean - (double)sh_part[1]);
+      }
     }
     __syncthreads();
     const float m0 = sh_part[0], m1 = sh_part[1], m2 = sh_part[2];
@@ -330,21 +346,21 @@ __global__ void __launch_bounds__(kBlock) normalize_kernel(const T *src, const i
       q.l += fmaf(2.f * d, e, fmaf(d, d, -p));
     }
     q.warp_reduce();
-    if (lane == 0) sh[warp] = q.value();
+    if (lane == 0) sh_pair[warp] = make_float2(q.h, q.l);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double var = 0.0;
-      for (int i = 0; i < kBlock / 32; ++i) var += sh[i];
-      var /= (double)n;
-      const double inv = 1.0 / sqrt(var + (double)eps);
-      sh_part[0] = (float)inv;
-      sh_part[1] = (float)(inv - (double)(float)inv);
-      sh[32] = var;
+    if (warp == 0) {
+      const double var = warps_total(sh_pair, lane) * rn;
+      const double inv = rsqrt(var + (double)eps);
+      if (lane == 0) {
+        sh_part[0] = (float)inv;
+        sh_part[1] = (float)(inv - (double)(float)inv);
+        sh_part[3] = (float)var;
+      }
     }
     __syncthreads();
     const float ih = sh_part[0], il = sh_part[1];
     // squares below the FP32 range (a deviation of 2^-60 and less next to no eps)
-    wild = sh[32] < 0x1p-80 && eps < 0x1p-60f;
+    wild = sh_part[3] < 0x1p-80f && eps < 0x1p-60f;
     if (!wild) {
 #pragma unroll 4
       for (int i = threadIdx.x; i < n; i += kBlock) {
