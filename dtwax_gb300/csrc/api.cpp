@@ -60,6 +60,11 @@ struct BatchCtx {
   HostBuf h_raw, h_meta, h_results, h_flags;
   int64_t seam_bytes = 0;
   bool meta_pending = false;
+  // Allocations so far of the buffers whose addresses a captured device batch holds.
+  uint64_t allocations() const {
+    return query.allocations + meta.allocations + keys.allocations + seam.allocations + flags.allocations +
+           h_meta.allocations;
+  }
 };
 
 struct ServeRead {
@@ -105,8 +110,12 @@ struct dtwx_handle {
   };
   std::map<std::tuple<int, int, int>, Tuned> tuned;
   Shape override_shape;      // set while the autotuner times a candidate
-  // CUDA graph of the most recent repeated device batch
-  uint64_t graph_key = 0, graph_pending = 0;
+  // CUDA graph of the most recent repeated device batch.  It holds the addresses
+  // of ctx[0]'s buffers and a launch shape, so it and the direct run before it
+  // count only while neither has changed: graph_plan, pending_plan are
+  // graph_plan_now() of their time
+  uint64_t graph_key = 0, graph_pending = 0, graph_plan = 0, pending_plan = 0;
+  uint64_t tunings = 0;  // autotuned shapes stored so far
   cudaGraphExec_t graph_exec = nullptr;
   int32_t graph_launches = 0;
   int64_t graph_replays = 0;
@@ -157,6 +166,10 @@ struct CaptureGuard {
   cudaStream_t st;
   ~CaptureGuard();
 };
+
+// Changes whenever a buffer of a captured batch is reallocated or a tuned shape is stored (both
+// terms only grow).
+uint64_t graph_plan_now(const dtwx_handle *h) { return h->ctx[0].allocations() + h->tunings; }
 
 #define CK(h, call)                                                                         \
   do {                                                                                      \
@@ -720,6 +733,12 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
     mix((uint64_t)precision);
     for (int r = 0; r <= n_reads; ++r) mix((uint64_t)offsets[r]);
     key = hsh | 1;
+    if (h->graph_exec && h->graph_plan != graph_plan_now(h)) {
+      // another call has since taken larger buffers, or a shape was tuned
+      cudaGraphExecDestroy(h->graph_exec);
+      h->graph_exec = nullptr;
+      h->graph_key = 0;
+    }
     if (key == h->graph_key && h->graph_exec) {
       // the pinned metadata blob was refilled above; the graph's copy reads it at replay
       CK(h, cudaGraphLaunch(h->graph_exec, st));
@@ -729,11 +748,12 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
       ++h->graph_replays;
       return DTWX_OK;
     }
-    if (key == h->graph_pending) {
+    if (key == h->graph_pending && h->pending_plan == graph_plan_now(h)) {
+      // (nothing is allocated under the capture: the direct run left every buffer large enough)
       CK(h, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
       h->capturing = true;
     } else {
-      h->graph_pending = key;
+      h->graph_pending = 0;  // until this direct run is through
     }
   }
   const void *src_dev = raw_dev;
@@ -842,10 +862,14 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
     if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
     h->graph_exec = exec;
     h->graph_key = key;
+    h->graph_plan = graph_plan_now(h);
     h->graph_launches = launches;
     CK(h, cudaGraphLaunch(exec, st));
     CK(h, cudaEventRecord(c.meta_free, st));
     c.meta_pending = true;
+  } else if (graphable) {
+    h->graph_pending = key;
+    h->pending_plan = graph_plan_now(h);
   }
   if (out_host) {
     // results and error word into pinned memory, one wait for both (a pageable
@@ -1328,6 +1352,7 @@ int dtwx_autotune(dtwx_handle *h, int32_t n_reads_req, int32_t read_len, float *
   const dtwx_handle::Tuned tw{win.S, win.warps, win.permille / 1000.0};
   h->tuned[std::make_tuple(prec, log2_bucket(n_reads_req), log2_bucket(read_len))] = tw;
   h->tuned[std::make_tuple(prec, log2_bucket(n_reads), log2_bucket(read_len))] = tw;
+  ++h->tunings;
   if (best_ms) *best_ms = best;
   return DTWX_OK;
 }

@@ -14,6 +14,7 @@ namespace dtwx {
 struct DevBuf {
   void *p = nullptr;
   size_t cap = 0;
+  uint64_t allocations = 0;  // so far: a captured graph holds the pointer of one of them
   cudaError_t ensure(size_t bytes) {
     if (bytes <= cap && p) return cudaSuccess;
     if (p) cudaFree(p);
@@ -22,6 +23,7 @@ struct DevBuf {
     size_t want = bytes < 256 ? 256 : bytes;
     cudaError_t e = cudaMalloc(&p, want);
     if (e == cudaSuccess) cap = want;
+    ++allocations;
     return e;
   }
   void release() {
@@ -36,6 +38,7 @@ struct DevBuf {
 struct HostBuf {
   void *p = nullptr;
   size_t cap = 0;
+  uint64_t allocations = 0;
   cudaError_t ensure(size_t bytes) {
     if (bytes <= cap && p) return cudaSuccess;
     if (p) cudaFreeHost(p);
@@ -44,6 +47,7 @@ struct HostBuf {
     size_t want = bytes < 4096 ? 4096 : bytes + bytes / 4;
     cudaError_t e = cudaMallocHost(&p, want);
     if (e == cudaSuccess) cap = want;
+    ++allocations;
     return e;
   }
   void release() {

@@ -83,7 +83,8 @@ typedef struct dtwx_config {
                               sweep the strips of a work item together */
   int32_t use_graphs;      /* 1: dtwx_classify_device replays a captured CUDA graph when a batch
                               repeats (same buffers, offsets and stream): the first such batch runs
-                              directly, the second is captured, later ones are replays */
+                              directly, the second is captured, later ones are replays, until another
+                              call makes the handle's buffers grow or dtwx_autotune stores a shape */
   int32_t serve_batches;   /* serving batches in flight at once (1..4), 0 = 2 */
   int32_t recurrence;      /* DTWX_NO_REF_DEL (default) or DTWX_REF_DEL */
   int32_t state_precision; /* DTWX_STATE_FP32 (default) or DTWX_STATE_FP16 */
