@@ -744,6 +744,8 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
       CK(h, cudaGraphLaunch(h->graph_exec, st));
       CK(h, cudaEventRecord(c.meta_free, st));
       c.meta_pending = true;
+      CK(h, cudaEventRecord(c.done, st));
+      h->device_call_pending = true;
       h->last_launches = h->graph_launches;
       ++h->graph_replays;
       return DTWX_OK;

@@ -73,3 +73,23 @@ def test_a_graph_ends_with_the_buffers_it_holds(case, kind):
     for got, _ in seen + after:
         for k in ("score_fwd", "score_rev", "end_pos", "strand", "call"):
             np.testing.assert_array_equal(got[k], want[k], err_msg=k)  # FP32: the same bits for every shape
+
+
+def test_sync_waits_for_a_replay(built_lib):
+    """dtwx_sync returns once the replayed kernels are through, as after a
+    direct call (the batch takes a few milliseconds)."""
+    import torch
+    import dtwax_gb300 as d
+    g = small_genome(200_000, 53)
+    tab = synth.level_table()
+    reads = reads_of_lengths(g, g, tab, [2000] * 200)
+    with make_classifier(g, tab, precision=d.FP16, use_graphs=1) as clf:
+        stream = torch.cuda.Stream()
+        raw = torch.tensor(reads.raw, device="cuda")
+        out = torch.zeros(32 * reads.n, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        for replays in (0, 0, 1, 2):
+            clf.classify_device(raw.data_ptr(), reads.offsets, out.data_ptr(), stream.cuda_stream)
+            clf.sync()
+            assert stream.query()
+            assert clf.tuning()["graph_replays"] == replays
