@@ -1373,12 +1373,12 @@ int dtwx_last_sweep_ms(dtwx_handle *h, float *ms) {
 int dtwx_get_tuning(const dtwx_handle *h, int32_t *out, int32_t n) {
   if (!h || !out || n < 0) return DTWX_E_ARG;
   const Shape &s = h->last_shape[h->cfg.precision];
-  const int32_t v[8] = {s.S, s.G, s.warps, s.grid, (int32_t)std::min<int64_t>(s.items, INT32_MAX),
+  const int32_t v[9] = {s.S, s.G, s.warps, s.grid, (int32_t)std::min<int64_t>(s.items, INT32_MAX),
                         s.S ? sdtw_ctas_per_sm(h->cfg.precision, s.S, s.warps,
                                                h->cfg.recurrence == DTWX_REF_DEL)
                             : 0,
-                        (int32_t)h->graph_replays, s.nh ? 1 : 0};
-  for (int i = 0; i < n && i < 8; ++i) out[i] = v[i];
+                        (int32_t)h->graph_replays, s.nh ? 1 : 0, s.deal ? 1 : 0};
+  for (int i = 0; i < n && i < 9; ++i) out[i] = v[i];
   return DTWX_OK;
 }
 

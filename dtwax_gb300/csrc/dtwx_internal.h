@@ -91,7 +91,8 @@ struct SdtwParams {
   int32_t narrow_halo;         // FP16 pairs: launch the instance with kNarrowHaloCells-wide halo strips
   int32_t team_warps;          // REF_DEL: warps that sweep an item's strips together (divides the CTA's warps;
                                // in the NO_REF_DEL kernels the CTA's warps are one team)
-  int32_t deal;                // 1: CTA b takes items b, b + grid, ...; 0: the next ticket of `counter`
+  int32_t deal;                // 1: CTA b takes items b, b + grid, ..., or with halo_read the b-th CTA to start
+                               // the b-th of grid consecutive parts; 0: the next ticket of `counter`
   uint64_t deal_warps;         // deal: the warp that takes the p-th strip of the CTA's first round, 4 bits each
   uint32_t spin_limit;         // polls before a bounded wait gives up; 0 = kSpinLimit
   int32_t stall_item;          // test hook: 1 + the queue ticket whose first reference-strip copy

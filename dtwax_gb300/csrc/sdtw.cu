@@ -544,15 +544,18 @@ __device__ __forceinline__ void save_row_state(const typename Pol<PREC>::V (&D)[
 
 // Wait until the resumed halos that start from the saved row of columns
 // [x, x + W) have read it: the halos of the chunks to the right of this one
-// that reach column x.  Those chunks were handed out before this one and their
-// halo strips depend on nothing of it.  Bounded like team_wait.
+// that reach column x.  Those chunks have lower item numbers: they were handed
+// out before this one (tickets), or belong to a CTA that started before this one
+// (ORDERED below), and their halo strips depend on nothing of it.  Bounded; it
+// gives up before the waits of team_wait that can be behind it (at a third of a
+// microsecond a poll or more: a tenth of a second and 5 us a row).
 template <int W, int WH>
 __device__ __forceinline__ bool wait_halo_readers(const SdtwParams &p, const Item &g, int64_t x, int item, int chunk,
                                                   int n, uint32_t abort_addr) {
   for (int c = chunk + 1; c < p.n_chunks; ++c) {
     const Item h = item_geometry<W, WH>(p, c, n);
     if (h.x0 >= x + W) break;
-    const uint32_t limit = (1u << 22) + 256u * (uint32_t)min(n, 1 << 23);
+    const uint32_t limit = (1u << 18) + 16u * (uint32_t)min(n, 1 << 23);
     bool done = false;
     for (uint32_t it = 0; it < limit && !done; ++it) {
       int32_t v;
@@ -789,7 +792,14 @@ __device__ __forceinline__ bool sweep_strip(const SdtwParams &p, const Strip &st
 // ST16: FP16 cells whose serving row state is FP16 (p.state_fp16); a separate
 // instance, so the other instances carry none of its registers.
 // NH: halo strips kNarrowHaloCells wide (FP16 pairs, p.narrow_halo).
-template <int S, int PREC, bool ST16, bool NH>
+// ORDERED: dealt batches that resume and save rows.  Their items wait for items
+// of lower number (wait_halo_readers), so a CTA's number is a ticket, taken when
+// it starts, and its items are consecutive: whatever it waits for is its own or
+// belongs to a CTA that started before it, and the wait ends even while another
+// kernel keeps the remaining CTAs off the GPU.  An instance of its own: its few
+// registers cost the others' rows 2 % (192 FP32 reads of 2,000 samples against
+// 1 Mb: 61.0 ms, 62.1 with it).
+template <int S, int PREC, bool ST16, bool NH, bool ORDERED>
 __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
     const __grid_constant__ CUtensorMap tmap, const SdtwParams p) {
   using P = Pol<PREC>;
@@ -804,6 +814,7 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
   // many items and whose rows lose 6 % to the registers of the first round
   constexpr bool DEAL = PREC != 0 || NH;
   static_assert(S % SH == 0 && SH % 8 == 0, "halo strips must tile the chunk start");
+  static_assert(!ORDERED || DEAL, "only a dealt batch has an order of CTAs");
   static_assert(!NH || PREC == 0, "narrow halo strips are built for FP16 pairs");
   static_assert(STRIP_BYTES % 1024 == 0, "strip tile must keep 1024-byte alignment");
   static_assert(S % 8 == 0, "row state and reference move in 16-byte groups");
@@ -840,7 +851,7 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
   uint32_t phase = 0;  // parity of the tile's next completion
 
   const uint32_t lock_a = team, abort_a = team + 4, item_a = team + 8, next_a = team + 12, total_a = team + 16,
-                 seq_a = team + 20, dealt_a = team + 24;
+                 seq_a = team + 20, dealt_a = team + 24, end_a = team + 28;
   const int64_t seam_half = p.seam_stride / 2;
   char *const seam_base = p.seam + (int64_t)blockIdx.x * nbuf * seam_half;
   // FP32 and MIXED split each (task, chunk) into one work item per strand
@@ -868,24 +879,41 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
   // lived through every row (4 reads of 1,600 samples against 5 Mb: 4.26 to
   // 4.22 ms).  FP32 and MIXED keep it in registers, which their schedule
   // takes better (192 reads of 2,000 samples against 1 Mb: 60.8 and 58.4 ms,
-  // 61.4 and 59.2 through shared memory).
-  constexpr bool FIRST_SHARED = PREC == 0;
+  // 61.4 and 59.2 through shared memory); an ordered deal of MIXED cells takes
+  // the word better (three steps of a read of 1,600 samples a step against
+  // 120 kb: 577 us, 633 in registers).
+  constexpr bool FIRST_SHARED = PREC == 0 || (ORDERED && PREC == 2);
   const uint32_t first_a = smem_u32(bar + 1);
   if constexpr (DEAL && FIRST_SHARED) st_shared_u64(first_a, 0);
   int first_item = -1, first_s = 0;
   uint32_t first_seq = 0;
-  if (DEAL && p.deal) {
+  if constexpr (ORDERED) {
+    if (warp == 0) {
+      const int64_t cta = __shfl_sync(FULL_MASK, ticket_if(p.counter, is0), 0);
+      st_shared_volatile(dealt_a, (uint32_t)(cta * n_items / gridDim.x));
+      st_shared_volatile(end_a, (uint32_t)((cta + 1) * n_items / gridDim.x));
+    }
+    __syncthreads();
+  }
+  if (DEAL && (ORDERED || p.deal)) {
     int pos = 0;
     while (pos < 15 && (int)((p.deal_warps >> (4 * pos)) & 15u) != warp) ++pos;
     int at = 0, total = 0, dealt = 0;
-    int64_t item = blockIdx.x;
-    for (; item < n_items; item += gridDim.x) {
+    int64_t item = blockIdx.x, end = n_items;
+    int step = gridDim.x;
+    if constexpr (ORDERED) {
+      item = ld_shared_volatile(dealt_a);
+      end = ld_shared_volatile(end_a);
+      step = 1;
+      __syncthreads();  // (every warp has read the first item)
+    }
+    for (; item < end; item += step) {
       ++dealt;
       total = item_strips((int)item);
       if (pos < at + total) break;
       at += total;
     }
-    if (item < n_items) {
+    if (item < end) {
       first_item = (int)item;
       first_s = pos - at;
       first_seq = (uint32_t)pos;
@@ -897,7 +925,7 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
       st_shared_volatile(next_a, (uint32_t)(first_s + 1));
       st_shared_volatile(total_a, (uint32_t)total);
       st_shared_volatile(seq_a, (uint32_t)nwarps);
-      st_shared_volatile(dealt_a, (uint32_t)dealt);
+      st_shared_volatile(dealt_a, (uint32_t)(ORDERED ? item + 1 : dealt));
     }
     if constexpr (FIRST_SHARED)  // (strips of a first round: at most 16)
       st_shared_u64(first_a, (uint64_t)(0x80000000u | first_seq << 8 | (uint32_t)first_s) << 32 | (uint32_t)first_item);
@@ -933,7 +961,13 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
       int total = (int)ld_shared_volatile(total_a);
       seq = ld_shared_volatile(seq_a);
       while (s >= total && item < n_items) {
-        if (DEAL && p.deal) {
+        if constexpr (ORDERED) {
+          item = (int)ld_shared_volatile(dealt_a);
+          if (item >= (int)ld_shared_volatile(end_a)) item = (int)n_items;
+          __syncwarp();
+          st_shared_volatile(dealt_a, (uint32_t)(item + 1));
+          __syncwarp();
+        } else if (DEAL && p.deal) {
           const uint32_t dealt = ld_shared_volatile(dealt_a);
           item = (int)(blockIdx.x + dealt * gridDim.x);
           __syncwarp();
@@ -1080,11 +1114,15 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
 
 // ---------------------------------------------------------------- instances / launch
 
-template <int S, int PREC, bool ST16 = false, bool NH = false>
+template <int S, int PREC, bool ST16 = false, bool NH = false, bool ORDERED = false>
 static cudaError_t launch_inst(int warps, int grid, const SdtwParams &p, const CUtensorMap *tmap,
                                cudaStream_t s) {
+  constexpr bool kDeals = PREC != 0 || NH;
+  if constexpr (kDeals && !ORDERED) {
+    if (p.deal && p.halo_read) return launch_inst<S, PREC, ST16, NH, true>(warps, grid, p, tmap, s);
+  }
   const size_t smem = sdtw_smem_bytes(PREC, S, warps);
-  auto fn = sdtw_kernel<S, PREC, ST16, NH>;
+  auto fn = sdtw_kernel<S, PREC, ST16, NH, ORDERED>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   CUtensorMap dummy;
@@ -1100,7 +1138,7 @@ template <int S, int PREC, bool ST16 = false, bool NH = false>
 static int occ_inst(int warps) {
   int n = 0;
   const size_t smem = sdtw_smem_bytes(PREC, S, warps);
-  auto fn = sdtw_kernel<S, PREC, ST16, NH>;
+  auto fn = sdtw_kernel<S, PREC, ST16, NH, false>;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, warps * kWarp, smem) != cudaSuccess) return 0;

@@ -24,8 +24,8 @@ struct TeamState {
   int32_t next;    // its next strip
   int32_t total;   // its strips
   uint32_t seq;    // strips handed out so far
-  int32_t dealt;   // items begun (p.deal)
-  uint32_t pad;
+  int32_t dealt;   // items begun (p.deal); in an ordered deal the CTA's next item
+  int32_t end;     // ordered deal: the item after the CTA's last
 };
 static_assert(sizeof(TeamState) == kTeamStateBytes, "shared-memory layout of the team");
 

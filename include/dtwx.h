@@ -287,7 +287,8 @@ int dtwx_autotune(dtwx_handle *h, int32_t n_reads, int32_t read_len, float *best
 /* Launch shape of the handle's most recent batched sweep in its precision:
  * out[0..n) = cells per thread, strips per work item, warps per CTA, CTAs,
  * work items, resident CTAs per SM, CUDA-graph replays so far, 1 if the
- * narrow-halo kernel instance ran (as many as n asks for, up to 8). */
+ * narrow-halo kernel instance ran, 1 if the items were shared out to the CTAs
+ * in advance (as many as n asks for, up to 9). */
 int dtwx_get_tuning(const dtwx_handle *h, int32_t *out, int32_t n);
 
 /* Measured issue-rate ceiling of the cell update on this device: a kernel that
