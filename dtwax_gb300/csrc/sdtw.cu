@@ -1114,6 +1114,18 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
 
 // ---------------------------------------------------------------- instances / launch
 
+// Lets an instance take the shared memory of its largest CTA.  The limit belongs
+// to the function on the device, not to a launch: every caller sets the same
+// value, so that threads with CTAs of different sizes do not take it from each
+// other between their call here and their launch.
+constexpr int kMostWarps = 16;
+template <int S, int PREC, typename F>
+static cudaError_t allow_smem(F fn) {
+  static_assert(kMostWarps * (kWarp * S * Pol<PREC>::RB + 512) + 2048 <= 227 * 1024, "shared memory of an SM");
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sdtw_smem_bytes(PREC, S, kMostWarps));
+}
+
 template <int S, int PREC, bool ST16 = false, bool NH = false, bool ORDERED = false>
 static cudaError_t launch_inst(int warps, int grid, const SdtwParams &p, const CUtensorMap *tmap,
                                cudaStream_t s) {
@@ -1123,7 +1135,7 @@ static cudaError_t launch_inst(int warps, int grid, const SdtwParams &p, const C
   }
   const size_t smem = sdtw_smem_bytes(PREC, S, warps);
   auto fn = sdtw_kernel<S, PREC, ST16, NH, ORDERED>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem<S, PREC>(fn);
   if (e != cudaSuccess) return e;
   CUtensorMap dummy;
   if (!tmap) {
@@ -1139,8 +1151,7 @@ static int occ_inst(int warps) {
   int n = 0;
   const size_t smem = sdtw_smem_bytes(PREC, S, warps);
   auto fn = sdtw_kernel<S, PREC, ST16, NH, false>;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return 0;
+  if (allow_smem<S, PREC>(fn) != cudaSuccess) return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, warps * kWarp, smem) != cudaSuccess) return 0;
   return n;
 }
@@ -1222,10 +1233,10 @@ static int query_ctas_per_sm(int precision, int cells_per_thread, int warps_per_
 // A property of the compiled instance on this GPU model, asked several times
 // per call while a shape is picked: the occupancy API is asked once.
 int sdtw_ctas_per_sm(int precision, int cells_per_thread, int warps_per_cta, bool ref_del) {
-  static std::atomic<int8_t> known[2][3][5][17];  // 0: not asked yet, else 1 + CTAs
+  static std::atomic<int8_t> known[2][3][5][kMostWarps + 1];  // 0: not asked yet, else 1 + CTAs
   const int c = cells_per_thread / 16;
   if (precision < 0 || precision > 2 || c < 1 || c > 4 || cells_per_thread != 16 * c || warps_per_cta < 1 ||
-      warps_per_cta > 16)
+      warps_per_cta > kMostWarps)
     return 0;
   std::atomic<int8_t> &k = known[ref_del ? 1 : 0][precision][c][warps_per_cta];
   int8_t v = k.load(std::memory_order_relaxed);
