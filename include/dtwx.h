@@ -275,12 +275,14 @@ int32_t dtwx_last_launch_count(const dtwx_handle *h);
 int dtwx_last_sweep_ms(dtwx_handle *h, float *ms);
 
 /* Autotuner: time the sweep on a synthetic batch of n_reads reads of read_len
- * samples (cut to at most 2,048 reads and about 1.2e13 cells) for every
- * compiled cells-per-thread instance, 4 and 8 warps per CTA (and, for REF_DEL,
- * the default teams), and half / once / twice the analytic
- * chunk width; the fastest shape is used from then on for
- * batches of n_reads reads of that length (log2 buckets of read count and
- * read length).  *best_ms gets its sweep time.  The reference fixes these at
+ * samples (cut to at most 2,048 reads and about 1.2e13 cells) in the default
+ * shape and for every compiled cells-per-thread instance, 4 and 8 warps per CTA
+ * (REF_DEL: and the default teams), with half / once / twice the analytic chunk
+ * width and, for FP32 and MIXED cells, the chunks that the default shape would
+ * have; the fastest shape is used from then on for batches of n_reads reads of
+ * that length (log2 buckets of read count and read length).  The default shape
+ * stays where it is more than 3 % ahead of all others.  *best_ms gets the sweep
+ * time of the shape that is used.  The reference fixes these at
  * compile time (SEGMENT_SIZE, BLOCK_NUM; src/include/common.hpp:64-79). */
 int dtwx_autotune(dtwx_handle *h, int32_t n_reads, int32_t read_len, float *best_ms);
 

@@ -1,0 +1,61 @@
+"""dtwx_autotune against the shape that a batch gets without it.
+
+The default shape is one of the candidates, so tuning cannot make a batch
+slower than the noise of two runs (3 %, here with room for a busy host: the
+cases below were 1.4 and 1.7 times slower tuned than untuned when only CTAs of
+4 and 8 warps with the chunks of the old model were tried).
+"""
+import numpy as np
+import pytest
+
+from gpu_util import make_classifier, reads_of_lengths, small_genome
+from dtwax_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("score_fwd", "score_rev", "end_pos", "strand")
+
+
+def sweep_ms(clf, reads):
+    ms = []
+    for _ in range(9):
+        res = clf.classify(raw=reads.raw, offsets=reads.offsets)
+        ms.append(clf.last_sweep_ms())
+    return res, float(np.median(ms[2:])), clf.tuning()
+
+
+@pytest.mark.parametrize("precision", [1, 2])
+@pytest.mark.parametrize("n,length,genome", [(1, 1600, 500_000), (10, 2048, 48_502), (6, 2000, 20_000), (3, 900, 30_000)])
+def test_tuned_is_not_slower_than_untuned(built_lib, precision, n, length, genome):
+    g, tab = small_genome(genome, 81), synth.level_table()
+    reads = reads_of_lengths(g, g, tab, [length] * n)
+    with make_classifier(g, tab, precision=precision) as clf:
+        want, before, _ = sweep_ms(clf, reads)
+        best = clf.autotune(n, length)
+        got, after, shape = sweep_ms(clf, reads)
+        clf.autotune(n, length)
+        again, twice, _ = sweep_ms(clf, reads)
+    print(f"untuned {before:.3f} ms, tuned {after:.3f} ({best:.3f} while tuning), tuned twice {twice:.3f}: {shape}")
+    assert after < 1.15 * before and twice < 1.15 * before
+    for res in (got, again):
+        for k in FIELDS:
+            np.testing.assert_array_equal(res[k], want[k], err_msg=k)  # FP32 path cost: any shape, the same bits
+
+
+@pytest.mark.parametrize("precision", [1, 2])
+def test_tuned_serving_keeps_the_bits(built_lib, precision):
+    """A tuned shape whose items are dealt (one per CTA) resumes and saves rows as any other."""
+    g, tab = small_genome(48_502, 82), synth.level_table()
+    raw = reads_of_lengths(g, g, tab, [4800]).raw
+    out = []
+    for tune in (False, True):
+        with make_classifier(g, tab, precision=precision, threshold=-1.0) as clf:
+            if tune:
+                clf.autotune(1, 1600)
+            clf.serve_start(max_in_flight=1, chunks_per_decision=3)
+            for k in range(3):
+                clf.submit_chunk(0, 1, raw[1600 * k:1600 * (k + 1)], is_last=k == 2)
+                clf.serve_step()
+                clf.serve_drain()
+            out.append([(d["score"], d["end_pos"], d["strand"], d["chunks"]) for d in clf.poll_decisions()])
+    assert len(out[0]) == 3 and out[0] == out[1]
