@@ -1318,7 +1318,9 @@ int dtwx_autotune(dtwx_handle *h, int32_t n_reads_req, int32_t read_len, float *
     x ^= x << 13, x ^= x >> 7, x ^= x << 17;
     v = (float)((double)(x >> 11) * (1.0 / 9007199254740992.0) * 3.4641016 - 1.7320508);  // mean 0, var 1
   }
-  DevBuf dq, dout;
+  struct Batch : DevBuf {  // given back however the call ends
+    ~Batch() { release(); }
+  } dq, dout;
   CK(h, dq.ensure(sizeof(float) * q.size()));
   CK(h, dout.ensure(sizeof(dtwx_result) * (size_t)n_reads));
   CK(h, cudaMemcpy(dq.p, q.data(), sizeof(float) * q.size(), cudaMemcpyHostToDevice));

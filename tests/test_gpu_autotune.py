@@ -59,3 +59,16 @@ def test_tuned_serving_keeps_the_bits(built_lib, precision):
                 clf.serve_drain()
             out.append([(d["score"], d["end_pos"], d["strand"], d["chunks"]) for d in clf.poll_decisions()])
     assert len(out[0]) == 3 and out[0] == out[1]
+
+
+def test_tuning_gives_its_memory_back(built_lib):
+    import torch
+    g, tab = small_genome(6_000, 83), synth.level_table()
+    with make_classifier(g, tab, precision=0) as clf:
+        clf.autotune(64, 100_000)  # 26 MB of reads
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        for _ in range(4):
+            clf.autotune(64, 100_000)
+        torch.cuda.synchronize()
+        assert torch.cuda.mem_get_info()[0] >= free - (8 << 20)
