@@ -598,7 +598,9 @@ int check_device_flags(dtwx_handle *h, BatchCtx &c, bool copied = false) {
   else
     CK(h, cudaMemcpy(f, c.flags.p, sizeof(f), cudaMemcpyDeviceToHost));
   if (f[4]) CK(h, cudaMemset(c.flags.as<int32_t>() + 4, 0, sizeof(int32_t)));  // reported once
-  if (f[4] & kErrTmaTimeout) return fail(h, DTWX_E_TIMEOUT, "device: TMA wait gave up");
+  if (f[4] & kErrWaitTimeout)
+    return fail(h, DTWX_E_TIMEOUT,
+                "device: a bounded wait gave up (for a copy, a neighbour's rows, their readers or the team's lock)");
   if (f[4] & kErrBadTask) return fail(h, DTWX_E_CAPACITY, "device: task longer than the seam buffers");
   return DTWX_OK;
 }
@@ -1579,7 +1581,7 @@ int harvest(dtwx_handle *h, int slot) {
   const int32_t dev_err = c.h_flags.as<int32_t>()[4];
   if (dev_err) {
     CK(h, cudaMemset(c.flags.as<int32_t>() + 4, 0, sizeof(int32_t)));
-    return fail(h, (dev_err & kErrTmaTimeout) ? DTWX_E_TIMEOUT : DTWX_E_CAPACITY, "device error flag in a serving batch");
+    return fail(h, (dev_err & kErrWaitTimeout) ? DTWX_E_TIMEOUT : DTWX_E_CAPACITY, "device error flag in a serving batch");
   }
   if (c.sweep_timed) {
     float ms = 0.f;

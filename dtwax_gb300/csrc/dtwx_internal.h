@@ -53,7 +53,7 @@ struct Task {
 static_assert(sizeof(Task) == 32, "Task layout");
 
 // Device error flags (bit mask in *err).
-constexpr int32_t kErrTmaTimeout = 1;
+constexpr int32_t kErrWaitTimeout = 1;  // any bounded wait: strip copy, seam window, buffer, halo readers, lock
 constexpr int32_t kErrBadTask = 2;
 // dtwx_result.call of every read of a call whose kernels set a device error
 // flag (DTWX_CALL_DEVICE_ERROR of include/dtwx.h).

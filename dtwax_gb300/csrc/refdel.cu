@@ -230,7 +230,7 @@ __global__ void __maxnreg__((refdel_reg_cap<PREC, S>())) sdtw_refdel_kernel(cons
     // -- the next strip of the team's sequence (its items one after the other)
     bool ok = team_lock(lock_a, abort_a, is0);
     if (!ok) {
-      atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
+      atomicOr(p.err, kErrWaitTimeout);  // every lane: same bit
       st_shared_volatile(abort_a, 1);
       return;
     }
@@ -400,7 +400,7 @@ __global__ void __maxnreg__((refdel_reg_cap<PREC, S>())) sdtw_refdel_kernel(cons
       if (done > 0) team_publish(prog_out, seq, (uint32_t)min(done, n));
     }
     if (!ok) {
-      atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
+      atomicOr(p.err, kErrWaitTimeout);  // every lane: same bit
       st_shared_volatile(abort_a, 1);
       return;
     }

@@ -952,7 +952,7 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
     }
     if (item < 0) {
       if (!team_lock(lock_a, abort_a, is0)) {
-        atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
+        atomicOr(p.err, kErrWaitTimeout);  // every lane: same bit
         st_shared_volatile(abort_a, 1);
         return;
       }
@@ -1104,7 +1104,7 @@ __global__ void __maxnreg__((sdtw_reg_cap<S, PREC>())) sdtw_kernel(
       }
     }
     if (!ok) {
-      atomicOr(p.err, kErrTmaTimeout);  // every lane: same bit
+      atomicOr(p.err, kErrWaitTimeout);  // every lane: same bit
       st_shared_volatile(abort_a, 1);
       return;
     }
