@@ -1379,10 +1379,13 @@ int dtwx_autotune(dtwx_handle *h, int32_t n_reads_req, int32_t read_len, float *
   h->autotuning = false;
   if (rc != DTWX_OK) return rc;
   CK(h, cudaStreamSynchronize(st));
-  // The default shape stays where it is clearly ahead; two runs of a sweep differ by up to 3 %.
-  // (FP32, one read of 1,600 samples against 500 kb: 0.206 ms, 0.356 in the fastest shape of 4 or
-  // 8 warps; 6 reads of 2,000 against 20 kb: 0.141 in both, 0.158 without the estimate's chunks.)
-  const bool keep = untuned < 0.97f * best;
+  // The default shape stays where it is clearly ahead; two runs of a short sweep differ by up to
+  // 3 %.  (FP32, one read of 1,600 samples against 500 kb: 0.206 ms, 0.356 in the fastest shape of
+  // 4 or 8 warps; 6 reads of 2,000 against 20 kb: 0.141 in both, 0.158 without the estimate's
+  // chunks.)  FP16 pairs keep it unless another is clearly ahead: other chunks round otherwise, and
+  // the equal reads of this batch do not decide so little.  (5 Mb, 266 reads of 4,500 samples here:
+  // default 682 ms, 4 warps 679, 8 warps 680; 8,192 reads of 1,000 to 8,000: 20.17, 20.21, 20.83 s.)
+  const bool keep = prec == 0 && !rd ? best > 0.98f * untuned : untuned < 0.97f * best;
   for (int n : {n_reads_req, n_reads}) {
     const auto bucket = std::make_tuple(prec, log2_bucket(n), log2_bucket(read_len));
     if (keep)

@@ -281,8 +281,9 @@ int dtwx_last_sweep_ms(dtwx_handle *h, float *ms);
  * width and, for FP32 and MIXED cells, the chunks that the default shape would
  * have; the fastest shape is used from then on for batches of n_reads reads of
  * that length (log2 buckets of read count and read length).  The default shape
- * stays where it is more than 3 % ahead of all others.  *best_ms gets the sweep
- * time of the shape that is used.  The reference fixes these at
+ * stays where it is more than 3 % ahead of all others, for FP16 cells (whose
+ * rounding follows the chunks) also where no other is more than 2 % ahead of it.
+ * *best_ms gets the sweep time of the shape that is used.  The reference fixes these at
  * compile time (SEGMENT_SIZE, BLOCK_NUM; src/include/common.hpp:64-79). */
 int dtwx_autotune(dtwx_handle *h, int32_t n_reads, int32_t read_len, float *best_ms);
 

@@ -24,7 +24,7 @@ def sweep_ms(clf, reads):
     return res, float(np.median(ms[2:])), clf.tuning()
 
 
-@pytest.mark.parametrize("precision", [1, 2])
+@pytest.mark.parametrize("precision", [0, 1, 2])
 @pytest.mark.parametrize("n,length,genome", [(1, 1600, 500_000), (10, 2048, 48_502), (6, 2000, 20_000), (3, 900, 30_000)])
 def test_tuned_is_not_slower_than_untuned(built_lib, precision, n, length, genome):
     g, tab = small_genome(genome, 81), synth.level_table()
@@ -37,7 +37,7 @@ def test_tuned_is_not_slower_than_untuned(built_lib, precision, n, length, genom
         again, twice, _ = sweep_ms(clf, reads)
     print(f"untuned {before:.3f} ms, tuned {after:.3f} ({best:.3f} while tuning), tuned twice {twice:.3f}: {shape}")
     assert after < 1.15 * before and twice < 1.15 * before
-    for res in (got, again):
+    for res in (got, again) if precision != 0 else ():  # (FP16 rounds by the chunks)
         for k in FIELDS:
             np.testing.assert_array_equal(res[k], want[k], err_msg=k)  # FP32 path cost: any shape, the same bits
 
