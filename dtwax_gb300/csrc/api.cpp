@@ -326,8 +326,9 @@ int default_team(int precision, int full, double mean_rows, int64_t items, int G
     // time); single warps do, at the price of a last round that is not full
     // (1,638 items of 2,048 rows: 1.33 ms against 1.49; 702: 0.92 against 0.77)
     const double w = std::ceil((double)items / (4.0 * sms));
-    const double alone = std::max(1.05 * 265.0, std::min(w, 3.0) * 217.0) * std::ceil(w / 3.0);
-    if (alone <= 1.4 * 217.0 * (double)items / (4.0 * sms)) return 1;
+    const RowCost &c = kFp16RowCost;
+    const double alone = std::max(1.05 * c.alone, std::min(w, 3.0) * c.shared) * std::ceil(w / 3.0);
+    if (alone <= 1.4 * c.shared * (double)items / (4.0 * sms)) return 1;
   }
   return items >= (int64_t)8 * sms * (full / 4) ? 4 : full;
 }
@@ -854,7 +855,7 @@ int classify_common(dtwx_handle *h, const void *raw_host, const void *raw_dev, i
       p.team_warps = sh.team;
       p.deal = sh.deal ? 1 : 0;
       p.deal_warps = sh.deal_warps;
-        const int ii = inst_index(precision, sh.S);
+      const int ii = inst_index(precision, sh.S);
       p.use_tma = h->tmap_ok[precision][ii] ? 1 : 0;
       CK(h, launch_sdtw(precision, sh.S, sh.warps, sh.grid, p, p.use_tma ? &h->tmap[precision][ii] : nullptr,
                         st));
@@ -1277,8 +1278,8 @@ int dtwx_normalize(dtwx_handle *h, const float *d_raw, const int64_t *offsets, i
   const char *dm = c.meta.as<char>();
   CK(h, launch_normalize(d_raw, 0, reinterpret_cast<const int64_t *>(dm + L.src_off),
                          reinterpret_cast<const int64_t *>(dm + L.dst_off),
-                         reinterpret_cast<const int32_t *>(dm + L.nsamp), nullptr, nullptr, n_reads, w.max_len, h->cfg.norm_eps,
-                         d_query, st));
+                         reinterpret_cast<const int32_t *>(dm + L.nsamp), nullptr, nullptr, n_reads, w.max_len,
+                         h->cfg.norm_eps, d_query, st));
   h->last_launches = 1;
   return DTWX_OK;
 }
@@ -1727,8 +1728,8 @@ int dtwx_serve_step(dtwx_handle *h) {
   int launches = 0;
   CK(h, launch_normalize(c.raw.p, 0, reinterpret_cast<const int64_t *>(dm + L.src_off),
                          reinterpret_cast<const int64_t *>(dm + L.dst_off),
-                         reinterpret_cast<const int32_t *>(dm + L.nsamp), nullptr, nullptr, nb, max_len, h->cfg.norm_eps,
-                         c.query.as<float>(), st));
+                         reinterpret_cast<const int32_t *>(dm + L.nsamp), nullptr, nullptr, nb, max_len,
+                         h->cfg.norm_eps, c.query.as<float>(), st));
   ++launches;
   double mean = (double)total / nb;
   if (int rc = enqueue_sweep(h, c, h->cfg.precision, st, c.query.as<float>(), reinterpret_cast<const Task *>(dm + L.tasks),

@@ -216,14 +216,21 @@ cudaError_t launch_build_reference(const char *d_seq, int64_t L, const double *d
 //
 // 64-bit accuracy without the FP64 pipe, which has 1/64 of the FP32 rate here
 // (2,048 reads of 1,000 to 8,000 samples, one dtwx_normalize call after the
-// other: 244 us with FP64 passes, 43 now; 11 us for the bytes): sums, deviations and products are unevaluated pairs of floats
+// other: 244 us with FP64 passes, now 49 on reads that come from HBM and 42 on
+// the same 37 MB again and again, which L2 holds; 11 us for the bytes): sums,
+// deviations and products are unevaluated pairs of floats
 // (error-free sums and FMA products, Knuth and Dekker), about 48 bits, and
 // the mean, variance and reciprocal root of a read are FP64 in one warp, with as
 // few instructions as they take: a warp's total converted by each warp, added by
-// one thread and divided twice cost 6 us of the 43, and a third of the time of
-// short reads (4,096 of 200 to 400 samples: 47 us, 31 now).  The
-// result is the FP64 value rounded to FP32 except where that lies within 2^-47
-// of a rounding boundary.  Reads with samples of 2^40 or more, none above 2^-40,
+// one thread and divided twice cost 6 us more, and a third of the time of
+// short reads (4,096 of 200 to 400 samples: 47 us, 32 now; 120 with FP64 passes).
+// Accuracy: the mean is good to about 2^-47 of its own size, which is an absolute
+// error of every result, so a value whose deviation is as small as 2^-22 of the
+// mean may miss the FP32 nearest to the 64-bit value; the largest error of a read
+// does not change.  (11 kinds of input, 200 to 40,000 samples, against 80 bits:
+// the same errors as with FP64 passes in 42 of 44; 592 of 2,000 values spread
+// 1e-5 about 90 rounded better, 986 of 40,000 spread 1 about 1e6 worse, by at most
+// 0.16 units.)  Reads with samples of 2^40 or more, none above 2^-40,
 // NaN or infinity, or a deviation whose squares leave the FP32 range take the
 // FP64 passes.  The samples of a read are read once and kept in shared memory
 // (up to kNormStaged of them).

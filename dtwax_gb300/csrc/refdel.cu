@@ -19,7 +19,8 @@
 // * lane 0 takes both from the seam column of the strip to the left, and lane
 //   31 writes the seam column for the strip to its right.
 // Each step a lane computes two consecutive rows, interleaved (two dependency
-// chains).  A cell costs one subtraction, two minima and one FMA.  A strip
+// chains).  A cell costs one subtraction, one three-input minimum (FP16 pairs: two
+// minima) and one FMA.  A strip
 // takes ceil(n / 2) + 31 steps; in the first and last 31 some lanes have no
 // rows and keep their cells, so after the last step every lane holds row
 // n - 1.
@@ -179,12 +180,13 @@ __device__ __forceinline__ void refdel_step(Lane<PREC, S> &L, int st, int n, int
   }
 }
 
-// FP32 at 16 cells per lane and FP16 pairs at 32 fit in 128 registers (16 warps
-// per SM); FP32 at 32 takes 12 warps rather than spill.
-template <int PREC, int S> constexpr int refdel_reg_cap() { return 128; }
+// 128 registers: 16 warps per SM, at the price of 40 to 60 bytes a thread spilled
+// outside the steps at 32 cells per lane.  (512 reads of 2,000 samples against
+// 48 kb, FP32 at 32 cells: 12.0 ms; 12.95 with 168 registers and 12 warps.)
+constexpr int kRefDelRegs = 128;
 
 template <int PREC, int S>
-__global__ void __maxnreg__((refdel_reg_cap<PREC, S>())) sdtw_refdel_kernel(const SdtwParams p) {
+__global__ void __maxnreg__(kRefDelRegs) sdtw_refdel_kernel(const SdtwParams p) {
   static_assert(S % 4 == 0, "row state moves in 16-byte groups");
   using C = Cells<PREC>;
   using V = typename C::V;

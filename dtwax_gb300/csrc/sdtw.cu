@@ -76,10 +76,9 @@ template <> struct Pol<0> {  // FP16 pairs
     memcpy(&v, &u, 4);
     return v;
   }
-  // query window: one half2 (q, q) per lane, broadcast by one shuffle per row
+  // a query sample as the cells take it: (q, q)
   using QW = __half2;
   __device__ __forceinline__ static QW qw(float q) { return __float2half2_rn(q); }
-  __device__ __forceinline__ static V qbcast(QW w, int il) { return __shfl_sync(FULL_MASK, w, il); }
 };
 
 template <> struct Pol<1> {  // FP32, one strand
@@ -101,7 +100,6 @@ template <> struct Pol<1> {  // FP32, one strand
   __device__ __forceinline__ static V from_bits(uint32_t u) { return __uint_as_float(u); }
   using QW = float;
   __device__ __forceinline__ static QW qw(float q) { return q; }
-  __device__ __forceinline__ static V qbcast(QW w, int il) { return __shfl_sync(FULL_MASK, w, il); }
 };
 
 template <> struct Pol<2> {  // MIXED: FP16 differences, FP32 path cost, one strand
@@ -119,7 +117,6 @@ template <> struct Pol<2> {  // MIXED: FP16 differences, FP32 path cost, one str
   __device__ __forceinline__ static V from_bits(uint32_t u) { return __uint_as_float(u); }
   using QW = __half2;
   __device__ __forceinline__ static QW qw(float q) { return __float2half2_rn(q); }
-  __device__ __forceinline__ static QW qbcast(QW w, int il) { return __shfl_sync(FULL_MASK, w, il); }
 };
 
 // d*d + c with d in FP16 and c, the result in FP32, one rounding (PTX
@@ -143,21 +140,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
 }
 
 // Bounded wait on an mbarrier phase: at most `limit` polls; false when the
@@ -176,16 +164,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32
     if (done) return true;
   }
   return false;
-}
-
-// 2-D tiled TMA load: box of the tensor map at (c0, c1) into shared memory.
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0,
-                                            int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-      : "memory");
 }
 
 // Lane-0 actions as predicated PTX: every lane executes the same instruction

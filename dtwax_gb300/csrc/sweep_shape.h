@@ -17,7 +17,8 @@ struct RowCost {
   int S;
   double alone, shared;
 };
-constexpr RowCost kRowCost[3][3] = {{{32, 250, 156}, {48, 265, 217}, {0, 0, 0}},
+constexpr RowCost kFp16RowCost = {48, 265, 217};  // (the estimate is of FP32 and MIXED shapes)
+constexpr RowCost kRowCost[3][3] = {{},
                                     {{16, 150, 65}, {32, 230, 111}, {48, 290, 152}},
                                     {{32, 260, 115}, {48, 320, 148}, {64, 360, 184}}};
 
@@ -27,8 +28,8 @@ constexpr RowCost kRowCost[3][3] = {{{32, 250, 156}, {48, 265, 217}, {0, 0, 0}},
 // 32-row window behind its left neighbour, and share the SM's schedulers; both
 // limits are real at once near the middle, so they add in squares (within 10 %
 // of 270 measured shapes of eight batches, FP32 and MIXED cells).
-inline double sweep_estimate(const RowCost &c, int64_t items, double work, double strips, double rows, int k, int64_t teams,
-                      int sms) {
+inline double sweep_estimate(const RowCost &c, int64_t items, double work, double strips, double rows, int k,
+                             int64_t teams, int sms) {
   const double per_team = std::ceil((double)items / (double)teams) * work;
   const double alone = c.alone * (rows * std::max(1.0, per_team / k) + kWarp * (std::min(strips, (double)k) - 1.0));
   const double ctas_per_sm = (double)teams / sms;

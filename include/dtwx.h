@@ -149,6 +149,11 @@ int dtwx_create_from_sequence(const dtwx_config *cfg, const float *level_table,
                               const char *seq, int64_t seq_len,
                               dtwx_handle **out);
 
+/* Frees what the handle owns.  One 256-byte device allocation per device, made
+ * by the first dtwx_create* there, stays until the process (or its context)
+ * ends: it keeps the block that the driver serves small requests from (2 MB)
+ * mapped, which otherwise every create and destroy of a small classifier would
+ * map and unmap.  Processes that share a GPU count it as theirs. */
 int dtwx_destroy(dtwx_handle *h);
 
 /* Text of the last failure on this handle (never NULL).  With h == NULL it
@@ -167,8 +172,8 @@ int dtwx_get_reference(dtwx_handle *h, float *fwd, float *rev);
  * device work.
  *
  * Classify reads given as raw FP32 samples on the host: read r is
- * raw[offsets[r] .. offsets[r+1]).  Window, z-score (FP64 statistics),
- * sDTW of both strands and the min/argmin all run on the GPU; out[n_reads] is
+ * raw[offsets[r] .. offsets[r+1]).  Window, z-score (statistics of about 48
+ * bits), sDTW of both strands and the min/argmin all run on the GPU; out[n_reads] is
  * written on return.  Replaces the batch loop of src/main.cu:217-271
  * (normalizer::normalize, src/include/normalizer.cu:370-413, then
  * FullDTW::distances per 10-read batch). */
@@ -207,7 +212,8 @@ int dtwx_classify_device(dtwx_handle *h, const float *d_raw, const int64_t *offs
  * of the handle's config (adapter_skip, query_len, require_full) of
  * d_raw[offsets[r] .. offsets[r+1]) (FP32 samples on the device, offsets on
  * the host) is z-scored per read, (x - mean) / sqrt(biased variance +
- * norm_eps) with FP64 statistics, into d_query (device), windows back to back.
+ * norm_eps) with statistics of about 48 bits (float pairs; FP64 for reads whose
+ * values leave their range), into d_query (device), windows back to back.
  * out_offsets (host, n_reads + 1 entries, may be NULL) receives where each
  * window starts in d_query and the total.  Asynchronous on `stream`.
  * Replaces normalizer::normalize (src/include/normalizer.cu:71-113), which

@@ -47,9 +47,9 @@ import concurrent.futures as cf
 import ctypes
 import os
 import subprocess
+import unittest
 
 import numpy as np
-import unittest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT_DIR = os.path.join(HERE, "_ref")
